@@ -686,8 +686,7 @@ def run_ours(args):
     # ---- per-phase profile at the end of the trajectory: primal roofline ---
     phases, info = w.profile_substep()
     lanes = tuned[0][0] if tuned else (args.lanes if args.lanes is not None else 1)
-    kind = "scene" if info["primal_launches"] == 1 and lanes < 0 else (
-        "split" if lanes <= 0 else ("thread" if lanes == 1 else "lanes"))
+    kind = "engine" if lanes <= 1 else "lanes"
     roof = roofline.primal_roofline(phases, info, hbm_peak(), kind=kind, iterations=params.iterations)
     roof["state"] = "one profiled substep at the end of the trajectory"
     # ---- e2e through the C ABI with host buffers, same trajectory steps ----

@@ -25,6 +25,7 @@
 // A body's update x1 = x + d, q1 = integrate(q, d_ang), d = -H^-1 r, has the
 // adjoint  s_bar = -(d(r + H d)/ds)^T H^-1 d_bar  for every input s; each
 // stamped row contributes through its force, penalty and lever.
+#define AVBD_PLAIN_DIV
 #include "avbd_common.cuh"
 #include "avbd_adjoint.cuh"
 

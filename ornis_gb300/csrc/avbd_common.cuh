@@ -424,13 +424,6 @@ static __device__ __forceinline__ int joint_members(const DW& w, uint32_t j, uin
     return 2;
 }
 
-// The body whose walk over its joints updates a joint's multipliers in the
-// per-scene solve: a joint's first body, a gear's first coupled body (a gear
-// is listed only on its coupled joints' bodies).
-static __device__ __forceinline__ uint32_t joint_dual_owner(const DW& w, uint32_t j) {
-    return w.j_kind[j] == AVBD_JOINT_GEAR ? w.j_ab[w.j_gb[j].x].x : w.j_ab[j].x;
-}
-
 // sleep.rs:30-105: how far a joint is from its assembly pose
 static __device__ __forceinline__ float joint_rest_error(const DW& w, uint32_t j) {
     if (w.j_kind[j] == AVBD_JOINT_GEAR) {

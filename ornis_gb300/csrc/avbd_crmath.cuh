@@ -264,6 +264,15 @@ CRM_HD uint32_t f2u(float f) {
     return u;
 #endif
 }
+CRM_HD float u2f(uint32_t u) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
+    float f;
+    std::memcpy(&f, &u, 4);
+    return f;
+#endif
+}
 CRM_HD bool sign_bit(float f) { return (f2u(f) >> 31) != 0u; }
 CRM_HD float next_up(float f) { return nextafterf(f, INFINITY); }
 CRM_HD float next_down(float f) { return nextafterf(f, -INFINITY); }
@@ -344,21 +353,28 @@ CRM_HD void two_sum_f(float a, float b, float& s, float& e) {
 // The value lies in [s + e - err, s + e + err], s = fl(s + e): s is its
 // correctly rounded float when neither end crosses the midpoint between s
 // and its neighbour on that side (the gaps below and above s differ at a
-// power of two).  The comparisons keep a 1% margin over the rounding of
-// e +- err.
+// power of two).  The comparisons keep a margin of 2^-20 over the rounding of
+// e +- err (a margin of 1% rejected 1% of all arguments).
 CRM_HD bool float_stage_ok(float s, float e, float err) {
 #ifdef AVBD_CRMATH_TEST_DOUBLE  // tests: skip the float stage
     return false;
 #else
     if (!(fabsf(s) < 3.0e38f) || fabsf(s) < 0x1p-100f) return false;
-    const float up = CRF_MUL(CRF_SUB(next_up(s), s), 0.5f);    // exact
-    const float dn = CRF_MUL(CRF_SUB(s, next_down(s)), 0.5f);  // exact
-    return CRF_MUL(CRF_ADD(e, err), 1.01f) < up && CRF_MUL(CRF_SUB(err, e), 1.01f) < dn;
+    // half the gap to the neighbour away from zero, and to the one towards it
+    const uint32_t u = f2u(s);
+    const float away = u2f((u & 0x7f800000u) - (24u << 23));
+    const float in = (u & 0x7fffffu) ? away : CRF_MUL(away, 0.5f);
+    const bool neg = (u >> 31) != 0u;
+    const float up = neg ? in : away, dn = neg ? away : in;
+    return CRF_MUL(CRF_ADD(e, err), 0x1.00001p+0f) < up && CRF_MUL(CRF_SUB(err, e), 0x1.00001p+0f) < dn;
 #endif
 }
 // x + x^3 (c1 + z (c2 + z c3)), z = x^2, |x| <= 1/16: the sin and asin
 // stages.  The series' next term is below 2^-36 |x|.
 CRM_HD bool odd_stage(float x, float c1, float c2, float c3, float& out) {
+#ifdef AVBD_CRMATH_TEST_FF  // tests: the float-float stage takes what it covers
+    return false;
+#endif
     const float z = CRF_MUL(x, x);
     const float p = CRF_FMA(CRF_FMA(c3, z, c2), z, c1);
     const float d = CRF_MUL(CRF_MUL(x, z), p);
@@ -373,6 +389,9 @@ CRM_HD bool sin_stage(float x, float& out) {
 }
 // 1 + z (-1/2 + z (1/24 - z/720)), |x| <= 1/16; next term below 2^-47
 CRM_HD bool cos_stage(float x, float& out) {
+#ifdef AVBD_CRMATH_TEST_FF
+    return false;
+#endif
     if (!(fabsf(x) <= 0.0625f)) return false;
     const float z = CRF_MUL(x, x);
     const float d = CRF_MUL(z, CRF_FMA(CRF_FMA(-0x1.6c16c2p-10f, z, 0x1.555556p-5f), z, -0.5f));
@@ -389,6 +408,9 @@ CRM_HD bool asin_stage(float x, float& out) {
 // atan2(y, x) for x > 0, |y| <= x/16: t = y/x = th + tl, atan(t) = t + t^3 (-1/3
 // + z (1/5 - z/7)); the next term is below 2^-35 |t|.
 CRM_HD bool atan2_stage(float y, float x, float& out) {
+#ifdef AVBD_CRMATH_TEST_FF
+    return false;
+#endif
     // y/x's remainder y - th x is exact only if it stays above the subnormal range
     if (!(x > 0.0f) || !(x < 3.0e38f) || !(fabsf(y) <= CRF_MUL(x, 0.0625f)) || fabsf(y) < 0x1p-90f) return false;
     const float th = CRF_DIV(y, x);
@@ -404,6 +426,119 @@ CRM_HD bool atan2_stage(float y, float x, float& out) {
     const float err = CRF_FMA(CRF_ADD(fabsf(tail), fabsf(tl)), 0x1p-20f, CRF_MUL(fabsf(th), 0x1p-31f));
     out = s;
     return float_stage_ok(s, e, err);
+}
+
+// ---- float-float stage ------------------------------------------------------------
+// What the float stage rejects, or does not cover, is evaluated on pairs of
+// floats (hi + lo, about 48 bits: Dekker, "A floating-point technique for
+// extending the available precision", Numer. Math. 18, 1971; the product's
+// rounding error from one FMA) before the double stage: the first two
+// Taylor terms as pairs, the rest of the series in float.  Settles all but
+// about 2^-10 of its arguments in about 80 float instructions, where the
+// double stage issues on a pipe of 1/64 the float rate.
+struct FF {
+    float hi, lo;
+};
+CRM_HD FF ff_quick(float a, float b) {  // |a| >= |b| or a == 0
+    const float s = CRF_ADD(a, b);
+    return {s, CRF_SUB(b, CRF_SUB(s, a))};
+}
+CRM_HD FF ff_prod(float a, float b) {  // exact
+    const float p = CRF_MUL(a, b);
+    return {p, CRF_FMA(a, b, -p)};
+}
+CRM_HD FF ff_mul(FF x, FF y) {
+    const float p = CRF_MUL(x.hi, y.hi);
+    float e = CRF_FMA(x.hi, y.hi, -p);
+    e = CRF_ADD(e, CRF_FMA(x.hi, y.lo, CRF_MUL(x.lo, y.hi)));
+    return ff_quick(p, e);
+}
+CRM_HD FF ff_add(FF x, FF y) {
+    float s, e;
+    two_sum_f(x.hi, y.hi, s, e);
+    return ff_quick(s, CRF_ADD(e, CRF_ADD(x.lo, y.lo)));
+}
+CRM_HD FF ff_neg(FF x) { return {-x.hi, -x.lo}; }
+CRM_HD FF ff_div(FF x, FF y) {
+    const float q = CRF_DIV(x.hi, y.hi);
+    // x - q y, the product split exactly
+    const FF p = ff_prod(q, y.hi);
+    const float r = CRF_ADD(CRF_ADD(CRF_SUB(x.hi, p.hi), CRF_SUB(x.lo, p.lo)), -CRF_MUL(q, y.lo));
+    return ff_quick(q, CRF_DIV(r, y.hi));
+}
+// first two coefficients of a series as pairs, the rest in float
+struct FFSeries {
+    FF c1, c2;
+};
+// z (c1 + z (c2 + z q)), q the rest of the series at z
+CRM_HD FF ff_tail(FF z, FFSeries c, float q) {
+    FF p = ff_add(c.c2, ff_quick(CRF_MUL(z.hi, q), 0.0f));
+    p = ff_add(c.c1, ff_mul(z, p));
+    return ff_mul(z, p);
+}
+// Round v, whose relative error is below 2^-42 (the pairs: a few 2^-46) plus
+// c z^3 (the float part, z^3 times its coefficient, a few float ulps).
+CRM_HD bool ff_round(FF v, float z, float c, float& out) {
+    out = v.hi;
+    return float_stage_ok(v.hi, v.lo, CRF_MUL(fabsf(v.hi), CRF_FMA(CRF_MUL(CRF_MUL(z, z), z), c, 0x1p-42f)));
+}
+// 2^-11 <= |x| < pi/4
+CRM_HD bool sin_ff(float x, float& out) {
+    const float ax = fabsf(x);
+    if (!(ax < 0.785398f) || ax < 0x1p-11f) return false;
+    const FF z = ff_prod(x, x);
+    const float q = CRF_FMA(CRF_FMA(CRF_FMA(0x1.612462p-33f, z.hi, -0x1.ae6456p-26f), z.hi, 0x1.71de3ap-19f), z.hi,
+                            -0x1.a01a02p-13f);
+    const FF t = ff_tail(z, FFSeries{{-0x1.555556p-3f, 0x1.555556p-28f}, {0x1.111112p-7f, -0x1.dddddep-32f}}, q);
+    return ff_round(ff_add(FF{x, 0.0f}, ff_mul(FF{x, 0.0f}, t)), z.hi, 0x1p-34f, out);
+}
+CRM_HD bool cos_ff(float x, float& out) {
+    const float ax = fabsf(x);
+    if (!(ax < 0.785398f) || ax < 0x1p-11f) return false;
+    const FF z = ff_prod(x, x);
+    const float q = CRF_FMA(CRF_FMA(CRF_FMA(-0x1.93974ap-37f, z.hi, 0x1.1eed9p-29f), z.hi, -0x1.27e4fcp-22f), z.hi, 0x1.a01a02p-16f);
+    const float q1 = CRF_FMA(q, z.hi, -0x1.6c16c2p-10f);
+    const FF t = ff_tail(z, FFSeries{{-0.5f, 0.0f}, {0x1.555556p-5f, -0x1.555556p-30f}}, q1);
+    return ff_round(ff_add(FF{1.0f, 0.0f}, t), z.hi, 0x1p-31f, out);
+}
+// 2^-11 <= |x| <= 1/4
+CRM_HD bool asin_ff(float x, float& out) {
+    const float ax = fabsf(x);
+    if (!(ax <= 0.25f) || ax < 0x1p-11f) return false;
+    const FF z = ff_prod(x, x);
+    float q = 0x1.3fde5p-7f;
+    q = CRF_FMA(q, z.hi, 0x1.7a8788p-7f);
+    q = CRF_FMA(q, z.hi, 0x1.c9999ap-7f);
+    q = CRF_FMA(q, z.hi, 0x1.1c4ec4p-6f);
+    q = CRF_FMA(q, z.hi, 0x1.6e8ba2p-6f);
+    q = CRF_FMA(q, z.hi, 0x1.f1c71cp-6f);
+    q = CRF_FMA(q, z.hi, 0x1.6db6dcp-5f);
+    const FF t = ff_tail(z, FFSeries{{0x1.555556p-3f, -0x1.555556p-28f}, {0x1.333334p-4f, -0x1.99999ap-29f}}, q);
+    return ff_round(ff_add(FF{x, 0.0f}, ff_mul(FF{x, 0.0f}, t)), z.hi, 0x1p-26f, out);
+}
+// atan2(y, x), both magnitudes well inside the float range
+CRM_HD bool atan2_ff(float y, float x, float& out) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
+    if (!(mx < 0x1p60f) || !(mn > 0x1p-40f) || !(mn > CRF_MUL(mx, 0x1p-11f))) return false;
+    const FF t = ff_div(FF{mn, 0.0f}, FF{mx, 0.0f});
+    const float k = rintf(CRF_MUL(t.hi, 4.0f));
+    const float c = CRF_MUL(k, 0.25f);
+    FF u = t;
+    if (k != 0.0f) u = ff_div(ff_add(t, FF{-c, 0.0f}), ff_add(FF{1.0f, 0.0f}, ff_mul(t, FF{c, 0.0f})));
+    const FF z = ff_mul(u, u);
+    float q = -0x1.745d18p-4f;
+    q = CRF_FMA(q, z.hi, 0x1.c71c72p-4f);
+    q = CRF_FMA(q, z.hi, -0x1.24924ap-3f);
+    FF v = ff_add(u, ff_mul(u, ff_tail(z, FFSeries{{-0x1.555556p-2f, 0x1.555556p-27f}, {0x1.99999ap-3f, -0x1.99999ap-29f}}, q)));
+    if (k == 1.0f) v = ff_add(FF{0x1.f5b76p-3f, -0x1.b4dfc8p-29f}, v);
+    else if (k == 2.0f) v = ff_add(FF{0x1.dac67p-2f, 0x1.586ed4p-28f}, v);
+    else if (k == 3.0f) v = ff_add(FF{0x1.4978fap-1f, 0x1.934f7p-28f}, v);
+    else if (k == 4.0f) v = ff_add(FF{0x1.921fb6p-1f, -0x1.777a5cp-26f}, v);
+    if (ay > ax) v = ff_add(FF{0x1.921fb6p+0f, -0x1.777a5cp-25f}, ff_neg(v));
+    if (sign_bit(x)) v = ff_add(FF{0x1.921fb6p+1f, -0x1.777a5cp-24f}, ff_neg(v));
+    if (sign_bit(y)) v = ff_neg(v);
+    return ff_round(v, z.hi, 0x1p-24f, out);
 }
 
 // ---- sin, cos -----------------------------------------------------------------
@@ -530,7 +665,7 @@ CRM_HD float sinf(float x) {
     if (!(fabsf(x) <= 3.4028235e38f)) return x - x;  // NaN for NaN and infinities
     if (x == 0.0f) return x;
     float f;
-    if (sin_stage(x, f)) return f;
+    if (sin_stage(x, f) || sin_ff(x, f)) return f;
     DD r;
     int j;
     reduce(x, r, j);
@@ -540,7 +675,7 @@ CRM_HD float cosf(float x) {
     if (!(fabsf(x) <= 3.4028235e38f)) return x - x;
     if (x == 0.0f) return 1.0f;
     float f;
-    if (cos_stage(x, f)) return f;
+    if (cos_stage(x, f) || cos_ff(x, f)) return f;
     DD r;
     int j;
     reduce(x, r, j);
@@ -557,7 +692,9 @@ CRM_HD void sincosf(float x, float* s, float* c) {
         return;
     }
     float fs, fc;
-    const bool ks = sin_stage(x, fs), kc = cos_stage(x, fc);
+    bool ks = sin_stage(x, fs), kc = cos_stage(x, fc);
+    if (!ks) ks = sin_ff(x, fs);
+    if (!kc) kc = cos_ff(x, fc);
     if (ks && kc) {
         *s = fs;
         *c = fc;
@@ -577,7 +714,7 @@ CRM_HD float asinf(float x) {
     if (!(ax <= 1.0f)) return (x - x) / (x - x);  // NaN for NaN and |x| > 1
     if (x == 0.0f) return x;
     float f;
-    if (asin_stage(x, f)) return f;
+    if (asin_stage(x, f) || asin_ff(x, f)) return f;
     const double sgn = x < 0.0f ? -1.0 : 1.0;
     const double a = (double)ax;
     double y;
@@ -639,7 +776,7 @@ CRM_HD float atan2f(float y, float x) {
         return xneg ? sy * dd_to_float(cst(C_PI)) : sy * 0.0f;
     }
     float f;
-    if (atan2_stage(y, x, f)) return f;
+    if (atan2_stage(y, x, f) || atan2_ff(y, x, f)) return f;
     const bool swap = ay > ax;
     const double num = swap ? (double)ax : (double)ay, den = swap ? (double)ay : (double)ax;
     const double t = CRM_DIV(num, den);  // [0, 1]

@@ -11,13 +11,11 @@
 namespace avbd {
 
 struct Tune {
-    int primal_lanes = 1;        // lanes cooperating on one body in the primal (1, 4, 8, 16, 32);
-                                 // 0: split primal (per (pair, side) rows, then per-body sums and solve);
-                                 // -1: per-scene solve (one block takes a scene through all
-                                 // iterations; split arithmetic; worlds with a scene above
-                                 // SCENE_MAX_BODIES run the split launches instead)
-    int primal_block = 128;      // threads per block of the primal kernel (per-scene solve: 128, 256, 512)
-    int primal_minb = 4;         // resident blocks per SM the thread-per-body primal is built for
+    int primal_lanes = 1;        // order in which a body's rows are summed: 1 row by row (the reference's),
+                                 // 0 and -1 pair by pair (the split order), all by the tile engine;
+                                 // 4, 8, 16, 32: that many lanes per body, one launch per colour
+    int primal_block = 128;      // threads per block of the lanes-per-body kernels
+    int primal_minb = 4;         // kept for callers that set it; the tile engine has one build
     int small_scene_max = 2048;  // scenes up to this many bodies use the one-CTA broadphase
     int sweep_rows = 1;          // larger scenes: 1 sweep per Morton-ordered cell row, 0 one x-sweep
     int fast = 0;                // 1: the fast build of the iteration kernels
@@ -37,6 +35,19 @@ size_t radix_hist_words(size_t n);
 // digit-major table (digit d of tile t at hist[d * ntiles + t]); returns ntiles
 int radix_pass(const uint32_t* keys, const uint32_t* vals, uint32_t* okeys, uint32_t* ovals, size_t n, int shift,
                uint32_t* hist, uint32_t* scan_tmp, cudaStream_t st);
+
+// Where the iterations of a substep record what the reverse sweep reads (null:
+// nothing is recorded): slices of an AdjFrame's arrays, slice it + 1 after
+// iteration it; qcap, slots: point entries and incidence slots the frame holds.
+struct IterRec {
+    float4* contrib = nullptr;
+    size_t cstride = 0;
+    uint32_t slots = 0;
+    float4 *pos = nullptr, *rot = nullptr, *lam = nullptr, *pen = nullptr;
+    size_t qstride = 0;
+    uint32_t qcap = 0;
+    float4* joint = nullptr;
+};
 
 // per substep phases
 void launch_begin_substep(const DW& w, cudaStream_t st);
@@ -72,8 +83,8 @@ void launch_events(const DW& w, int emit, int triggers, uint32_t* scan_tmp, cuda
     void launch_finish_substep(const DW& w, cudaStream_t st);                                             \
     void launch_primal_colour(const DW& w, const Tune& tune, int colour, uint32_t max_bodies, cudaStream_t st); \
     void launch_dual(const DW& w, const Tune& tune, cudaStream_t st);                                   \
-    void launch_solve_prep(const DW& w, const Tune& tune, cudaStream_t st);                               \
-    void launch_scene_solve(const DW& w, const Tune& tune, cudaStream_t st);
+    void launch_side_lists(const DW& w, cudaStream_t st);                                                 \
+    void launch_iterations(const DW& w, const Tune& tune, const IterRec& rec, cudaStream_t st);
 namespace exact {
 AVBD_SOLVE_DECLS
 }
@@ -92,19 +103,17 @@ inline void launch_primal_colour(const DW& w, const Tune& t, int c, uint32_t max
     if (t.fast) fast::launch_primal_colour(w, t, c, maxb, st);
     else exact::launch_primal_colour(w, t, c, maxb, st);
 }
-inline void launch_solve_prep(const DW& w, const Tune& t, cudaStream_t st) {
-    if (t.fast) fast::launch_solve_prep(w, t, st);
-    else exact::launch_solve_prep(w, t, st);
+inline void launch_side_lists(const DW& w, const Tune& t, cudaStream_t st) {
+    if (t.fast) fast::launch_side_lists(w, st);
+    else exact::launch_side_lists(w, st);
 }
-// every iteration of the substep by the per-scene solve (one launch)
-inline void launch_scene_solve(const DW& w, const Tune& t, cudaStream_t st) {
-    if (t.fast) fast::launch_scene_solve(w, t, st);
-    else exact::launch_scene_solve(w, t, st);
+// every iteration of the substep by the tile engine
+inline void launch_iterations(const DW& w, const Tune& t, cudaStream_t st, const IterRec& rec = IterRec{}) {
+    if (t.fast) fast::launch_iterations(w, t, rec, st);
+    else exact::launch_iterations(w, t, rec, st);
 }
-// the per-scene solve runs when chosen and every scene fits a block
-inline bool use_scene_solve(const DW& w, const Tune& t) {
-    return t.primal_lanes < 0 && w.max_scene <= (uint32_t)SCENE_MAX_BODIES;
-}
+// the tile engine runs: one launch takes every iteration
+inline bool use_engine(const Tune& t) { return t.primal_lanes <= 1; }
 inline void launch_dual(const DW& w, const Tune& t, cudaStream_t st) {
     if (t.fast) fast::launch_dual(w, t, st);
     else exact::launch_dual(w, t, st);

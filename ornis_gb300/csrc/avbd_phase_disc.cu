@@ -318,6 +318,7 @@ static __device__ __forceinline__ void build_pair(const DW& w, uint32_t p, uint2
     }
     w.p_ab[p] = ab;
     w.p_n[p] = st3(normal, sgn);
+    w.p_t1[p] = st3(tangent_t1(normal), 0.0f);  // the friction frame of the iterations (this pair's witnesses are read)
     w.p_mu[p] = make_float2(mu, mu);
     w.p_np[p] = (uint32_t)nf;
     if (w.p_old) w.p_old[p] = d.exists ? d.old : -1;

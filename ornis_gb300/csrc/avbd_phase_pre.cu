@@ -23,6 +23,7 @@ __global__ void k_begin(DW w) {
         w.ctr[C_POINTS] = 0;
         w.ctr[C_SLEEP] = 0;
         w.ctr[C_CCD_HITS] = 0;
+        w.ctr[C_ROLL] = 0;
         if (w.evs) w.evs[EV_TRIG_NOW] = 0;
     }
 }

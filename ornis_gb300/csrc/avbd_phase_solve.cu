@@ -20,8 +20,7 @@
 namespace avbd {
 namespace AVBD_SOLVE_NS {
 
-static __device__ __forceinline__ void load_ctx(const DW& w, uint32_t p, PairCtx& c) {
-    uint2 ab = w.p_ab[p];
+static __device__ __forceinline__ void load_ctx(const DW& w, uint32_t p, uint2 ab, PairCtx& c) {
     float4 n4 = w.p_n[p];
     c.a = ab.x;
     c.b = ab.y;
@@ -45,70 +44,148 @@ static __device__ __forceinline__ void load_ctx(const DW& w, uint32_t p, PairCtx
     c.sph_b = info_shape(__float_as_uint(b2.w)) == AVBD_SHAPE_SPHERE;
     c.rad_a = a0.w;
     c.rad_b = b0.w;
-    float4 ma = w.mat[c.a], mb = w.mat[c.b];
+    c.t1 = ld3(w.p_t1[p]);
+    c.t2 = cross(c.t1, c.n);
+}
+// the pair's rolling and torsion friction
+static __device__ __forceinline__ void load_rolling(const DW& w, PairCtx& c) {
+    const float4 ma = w.mat[c.a], mb = w.mat[c.b];
     c.mu_roll = fmaxf(ma.z, mb.z);
     c.mu_spin = fmaxf(ma.w, mb.w);
-    if (c.gap <= 0.0f) {
-        c.t1 = tangent_t1(c.n);
-        c.t2 = cross(c.t1, c.n);
-    }
+}
+static __device__ __forceinline__ void load_ctx(const DW& w, uint32_t p, PairCtx& c) {
+    load_ctx(w, p, w.p_ab[p], c);
+    load_rolling(w, c);
 }
 
-// Rows of point k of pair p for the body on side is_a (assembly.rs:99-252).
-static __device__ __forceinline__ void stamp_point(const DW& w, const PairCtx& c, uint32_t p, uint32_t k, bool is_a,
-                                                   Sys& s) {
-    uint32_t q = p * MAX_PTS + k;
-    float4 ra = w.q_ra[q], rb = w.q_rb[q];
-    float4 lam = w.q_lam[q];
-    float sign = is_a ? 1.0f : -1.0f;
-    bool touching = c.gap <= 0.0f;
-    float c0 = touching ? lam.w : 0.0f;
-    V3 rup, rlo;
-    contact_levers(c, ra, rb, rup, rlo);
-    float cn = row_c_levers(c, c.n, c0, rup, rlo);
-    V3 r_side = is_a ? rup : rlo;
-    if (!touching) {
+// Where a body's rows go.  Sys adds each row to the body's 6x6 system in a
+// thread's registers (stamp_row, stamp_angular in avbd_rows.cuh); RowSink
+// stages three of them, [first, first + 3) in stamping order, in an item's
+// shared-memory slot for the lanes that sum them.
+//
+// A slot holds three rows side by side: 8 float4, component k of which belongs
+// to row k: direction x y z, penalty, lever torque x y z, force.
+enum { ROW_NONE = 0, ROW_FULL = 1, ROW_ANG = 2, ROW_DIAG = 3 };  // 2 bits per row of a slot
+struct RowSink {
+    float* slot;
+    int first, n;     // rows staged elsewhere before these; rows seen
+    uint32_t types;
+};
+static __device__ __forceinline__ void put_row(RowSink& s, uint32_t type, V3 nn, float pen, V3 t, float f) {
+    const int k = s.n++ - s.first;
+    if (k < 0 || k >= 3) return;
+    float* o = s.slot + k;
+    o[0] = nn.x; o[4] = nn.y; o[8] = nn.z; o[12] = pen;
+    o[16] = t.x; o[20] = t.y; o[24] = t.z; o[28] = f;
+    s.types |= type << (2 * k);
+}
+static __device__ __forceinline__ void stamp_row(RowSink& s, V3 axis, float pen, float f, V3 r, float sign) {
+    V3 nn = sign * axis;
+    put_row(s, ROW_FULL, nn, pen, cross(r, nn), f);
+}
+static __device__ __forceinline__ void stamp_angular(RowSink& s, V3 g, float pen, float f) {
+    put_row(s, ROW_ANG, V0(), pen, g, f);
+}
+// a joint's geometric stiffness on the angular diagonal
+static __device__ __forceinline__ void stamp_diag(Sys& s, V3 d) {
+    s.h[tri(3, 3)] += d.x;
+    s.h[tri(4, 4)] += d.y;
+    s.h[tri(5, 5)] += d.z;
+}
+static __device__ __forceinline__ void stamp_diag(RowSink& s, V3 d) { put_row(s, ROW_DIAG, V0(), 0.0f, d, 0.0f); }
+
+// A point's levers and constraint values at the bodies' poses: the normal
+// row's, and with `friction` the tangent rows'.
+struct ContactGeo {
+    V3 rup, rlo, raf, rbf;
+    float cn, ct1, ct2;
+};
+static __device__ __forceinline__ ContactGeo contact_geo(const PairCtx& c, float4 ra, float4 rb, float c0, bool friction) {
+    ContactGeo g;
+    contact_levers(c, ra, rb, g.rup, g.rlo);
+    g.cn = row_c_levers(c, c.n, c0, g.rup, g.rlo);
+    g.raf = g.rup;
+    g.rbf = g.rlo;
+    g.ct1 = g.ct2 = 0.0f;
+    if (friction) {
+        friction_levers(c, g.rup, g.rlo, g.raf, g.rbf);
+        g.ct1 = row_c_levers(c, c.t1, 0.0f, g.raf, g.rbf);
+        g.ct2 = row_c_levers(c, c.t2, 0.0f, g.raf, g.rbf);
+    }
+    return g;
+}
+// Contact rows of a point for the body on side is_a (assembly.rs:99-252).
+// live: bit k, row k is stamped (rows: normal, two tangents; a separated pair
+// at most its damper as row 0).
+struct ContactRows {
+    uint32_t live;
+    float pen[3], f[3];
+    V3 lever, lever_f;  // of the normal row, of the tangent rows
+};
+static __device__ __forceinline__ ContactRows contact_rows(const DW& w, const PairCtx& c, const ContactGeo& g, bool is_a,
+                                                           float4 lam, float4 pen) {
+    ContactRows o;
+    o.live = 0u;
+    o.f[0] = o.f[1] = o.f[2] = 0.0f;
+    o.pen[0] = pen.x;
+    o.pen[1] = pen.y;
+    o.pen[2] = pen.z;
+    o.lever = is_a ? g.rup : g.rlo;
+    o.lever_f = is_a ? g.raf : g.rbf;
+    if (c.gap > 0.0f) {
         // separated damper, imminence-gated (assembly.rs:113-175)
         float approach = fmaxf(dot(ld3(w.vel[c.b]) - ld3(w.vel[c.a]), c.n), 0.0f);
-        if (c.gap - approach * w.dt > 0.0f) return;
-        if (fabsf(cn) >= C_EPS) {
+        if (c.gap - approach * w.dt > 0.0f) return o;
+        if (fabsf(g.cn) >= C_EPS) {
             float npts = (float)max(c.np, 1u);
             float ka = is_dynamic(w, c.a) ? w.inv_mass[c.a] : 0.0f;
             float kb = is_dynamic(w, c.b) ? w.inv_mass[c.b] : 0.0f;
             float m_red = ka + kb > NEAR_ZERO ? 1.0f / (ka + kb) : 0.0f;
             if (m_red > 0.0f) {
                 float pen_d = fminf(2.0f * m_red / (w.dt * w.dt) / npts, PENALTY_MAX);
-                stamp_row(s, c.n, pen_d, fminf(pen_d * cn, 0.0f), r_side, sign);
+                o.pen[0] = pen_d;
+                o.f[0] = fminf(pen_d * g.cn, 0.0f);
+                o.live = 1u;
             }
         }
-        return;
+        return o;
     }
-    const V3 t1 = c.t1, t2 = c.t2;
-    V3 raf, rbf;
-    friction_levers(c, rup, rlo, raf, rbf);
-    V3 r_side_f = is_a ? raf : rbf;
-    float ct1 = row_c_levers(c, t1, 0.0f, raf, rbf);
-    float ct2 = row_c_levers(c, t2, 0.0f, raf, rbf);
-    float4 pen = w.q_pen[q];
-    float f[3];
-    contact_force(cn, pen, lam, ct1, ct2, c.mu, f);
-    if (row_live(cn, f[0])) stamp_row(s, c.n, pen.x, f[0], r_side, sign);
-    if (row_live(ct1, f[1])) stamp_row(s, t1, pen.y, f[1], r_side_f, sign);
-    if (row_live(ct2, f[2])) stamp_row(s, t2, pen.z, f[2], r_side_f, sign);
+    if (!(c.gap <= 0.0f)) return o;
+    contact_force(g.cn, pen, lam, g.ct1, g.ct2, c.mu, o.f);
+    o.live = (row_live(g.cn, o.f[0]) ? 1u : 0u) | (row_live(g.ct1, o.f[1]) ? 2u : 0u) | (row_live(g.ct2, o.f[2]) ? 4u : 0u);
+    return o;
+}
+// Rolling and torsion rows of a touching point of normal force fn.
+template <class SINK>
+static __device__ __forceinline__ void stamp_rolling(const DW& w, const PairCtx& c, uint32_t q, bool is_a, float fn,
+                                                     SINK& s) {
     const float mu_roll = c.mu_roll, mu_spin = c.mu_spin;
-    if (mu_roll > 0.0f || mu_spin > 0.0f) {
-        V3 wrel = c.dra - c.drb;
-        float4 rl = w.q_roll[q];
-        V3 rax[3] = {t1, t2, c.n};
-        float murs[3] = {mu_roll, mu_roll, mu_spin};
-        float rls[3] = {rl.x, rl.y, rl.z};
-        for (int li = 0; li < 3; li++) {
-            if (murs[li] <= 0.0f) continue;
-            float cap = murs[li] * fabsf(f[0]);
-            float fr = fclamp(ROLL_PEN * dot(wrel, rax[li]) + rls[li], -cap, cap);
-            stamp_angular(s, is_a ? rax[li] : -rax[li], ROLL_PEN, fr);
-        }
+    V3 wrel = c.dra - c.drb;
+    float4 rl = w.q_roll[q];
+    V3 rax[3] = {c.t1, c.t2, c.n};
+    float murs[3] = {mu_roll, mu_roll, mu_spin};
+    float rls[3] = {rl.x, rl.y, rl.z};
+#pragma unroll
+    for (int li = 0; li < 3; li++) {
+        if (murs[li] <= 0.0f) continue;
+        float cap = murs[li] * fabsf(fn);
+        float fr = fclamp(ROLL_PEN * dot(wrel, rax[li]) + rls[li], -cap, cap);
+        stamp_angular(s, is_a ? rax[li] : -rax[li], ROLL_PEN, fr);
     }
+}
+// Rows of point k of pair p for the body on side is_a.
+static __device__ __forceinline__ void stamp_point(const DW& w, const PairCtx& c, uint32_t p, uint32_t k, bool is_a,
+                                                   Sys& s) {
+    const uint32_t q = p * MAX_PTS + k;
+    const float4 lam = w.q_lam[q];
+    const bool touching = c.gap <= 0.0f;
+    const ContactGeo g = contact_geo(c, w.q_ra[q], w.q_rb[q], touching ? lam.w : 0.0f, touching);
+    const ContactRows r = contact_rows(w, c, g, is_a, lam, w.q_pen[q]);
+    const float sign = is_a ? 1.0f : -1.0f;
+    if (r.live & 1u) stamp_row(s, c.n, r.pen[0], r.f[0], r.lever, sign);
+    if (r.live & 2u) stamp_row(s, c.t1, r.pen[1], r.f[1], r.lever_f, sign);
+    if (r.live & 4u) stamp_row(s, c.t2, r.pen[2], r.f[2], r.lever_f, sign);
+    if (c.gap <= 0.0f && (c.mu_roll > 0.0f || c.mu_spin > 0.0f)) stamp_rolling(w, c, q, is_a, r.f[0], s);
 }
 
 // Joint rows for body h (assembly.rs:255-881): Ball, Revolute (and its
@@ -119,7 +196,8 @@ static __device__ __forceinline__ void stamp_point(const DW& w, const PairCtx& c
 // (assembly.rs:426-454 slides, :650-682 hinges): the shared force on the
 // position-level row C = coord_a + ratio coord_b - constant, the slide
 // sides first, then the hinge sides.
-static __device__ __forceinline__ void stamp_gear(const DW& w, uint32_t j, uint32_t h, Sys& s) {
+template <class SINK>
+static __device__ __forceinline__ void stamp_gear(const DW& w, uint32_t j, uint32_t h, SINK& s) {
     const GearSide sd[2] = {gear_side(w, j, 0), gear_side(w, j, 1)};
     const float c = gear_error(w, j, sd[0], sd[1]);
     const float pen = w.j_pen_l[j].x;
@@ -139,8 +217,8 @@ static __device__ __forceinline__ void stamp_gear(const DW& w, uint32_t j, uint3
     }
 }
 
-template <bool ALL>
-static __device__ __forceinline__ void stamp_joint(const DW& w, uint32_t j, uint32_t h, Sys& s) {
+template <bool ALL, class SINK>
+static __device__ __forceinline__ void stamp_joint(const DW& w, uint32_t j, uint32_t h, SINK& s) {
     uint2 ab = w.j_ab[j];
     const uint32_t kind = w.j_kind[j];
     if (ALL && kind == AVBD_JOINT_GEAR) {
@@ -303,9 +381,8 @@ static __device__ __forceinline__ void stamp_joint(const DW& w, uint32_t j, uint
             for (int x = 0; x < 3; x++)
                 for (int y = 0; y < 3; y++) hm[x][y] += g[x][y] * fl[k];
         }
-        s.h[tri(3, 3)] += len(V3{hm[0][0], hm[1][0], hm[2][0]});
-        s.h[tri(4, 4)] += len(V3{hm[0][1], hm[1][1], hm[2][1]});
-        s.h[tri(5, 5)] += len(V3{hm[0][2], hm[1][2], hm[2][2]});
+        stamp_diag(s, V3{len(V3{hm[0][0], hm[1][0], hm[2][0]}), len(V3{hm[0][1], hm[1][1], hm[2][1]}),
+                         len(V3{hm[0][2], hm[1][2], hm[2][2]})});
     }
     // angular rows (a wheel's pair keys on its axle, in the weld-reference slots)
     if (kind == AVBD_JOINT_REVOLUTE || k_pri || k_whl) {
@@ -396,78 +473,71 @@ static __device__ __forceinline__ void stamp_joint(const DW& w, uint32_t j, uint
     }
 }
 
-// inertial block and rhs (assembly.rs:74-96)
-static __device__ __forceinline__ void inertial_block(const DW& w, uint32_t h, Sys& s) {
-    float dt2 = w.dt * w.dt;
+// inertial block and rhs (assembly.rs:74-96); rdt2: the reciprocal of dt^2,
+// shared by the block's ten divisions
+static __device__ __forceinline__ Recip recip_dt2(const DW& w) {
+    bool bad = false;
+    return recip_of(w.dt * w.dt, bad);
+}
+static __device__ __forceinline__ float div_dt2(float a, const Recip& r) {
+    bool bad = !(r.b >= 0x1p-40f && r.b <= 0x1p40f);
+    const float q = div_by(a, r, bad);
+    return bad ? a / r.b : q;
+}
+static __device__ __forceinline__ void inertial_block(const DW& w, uint32_t h, const Recip& rdt2, Sys& s) {
+    const float4 rot4 = w.rot[h], in4 = w.inertia[h], pos4 = w.pos[h], y4 = w.inertial[h], qt4 = w.inertial_rot[h];
     float im = is_dynamic(w, h) ? w.inv_mass[h] : 0.0f;
-    float m_dt2 = 1.0f / im / dt2;
+    float m_dt2 = div_dt2(1.0f / im, rdt2);
     float iw[3][3];
-    Q q = ldq(w.rot[h]);
-    world_inertia(ld3(w.inertia[h]), q, iw);
+    Q q = ldq(rot4);
+    world_inertia(ld3(in4), q, iw);
     for (int i = 0; i < 21; i++) s.h[i] = 0.0f;
     s.h[tri(0, 0)] = m_dt2;
     s.h[tri(1, 1)] = m_dt2;
     s.h[tri(2, 2)] = m_dt2;
     for (int a = 0; a < 3; a++)
-        for (int b = 0; b <= a; b++) s.h[tri(3 + a, 3 + b)] = iw[a][b] / dt2;
-    V3 rl = m_dt2 * (ld3(w.pos[h]) - ld3(w.inertial[h]));
+        for (int b = 0; b <= a; b++) s.h[tri(3 + a, 3 + b)] = div_dt2(iw[a][b], rdt2);
+    V3 rl = m_dt2 * (ld3(pos4) - ld3(y4));
     s.r[0] = rl.x;
     s.r[1] = rl.y;
     s.r[2] = rl.z;
-    V3 ra = mat3_vec(iw, quat_diff_vec(q, ldq(w.inertial_rot[h]))) / dt2;
-    s.r[3] = ra.x;
-    s.r[4] = ra.y;
-    s.r[5] = ra.z;
+    V3 ra = mat3_vec(iw, quat_diff_vec(q, ldq(qt4)));
+    s.r[3] = div_dt2(ra.x, rdt2);
+    s.r[4] = div_dt2(ra.y, rdt2);
+    s.r[5] = div_dt2(ra.z, rdt2);
 }
 
-static __device__ __forceinline__ void apply_solve(const DW& w, uint32_t h, const Sys& s) {
+// What a body's update reads besides its system, loaded ahead of the solve.
+struct BodyPose {
+    float4 pos, rot, pos0, rot0;
+    float par;      // first shape parameter
+    uint32_t info;
+};
+static __device__ __forceinline__ BodyPose load_pose(const DW& w, uint32_t h) {
+    return BodyPose{w.pos[h], w.rot[h], w.pos0[h], w.rot0[h], w.shp[h].x, w.info[h]};
+}
+static __device__ __forceinline__ void apply_solve(const DW& w, uint32_t h, const BodyPose& b, const Sys& s) {
     float dx[6];
-    if (solve_6x6(s, dx)) {
-        V3 p = ld3(w.pos[h]) + V3{dx[0], dx[1], dx[2]};
-        Q q = quat_integrate(ldq(w.rot[h]), V3{dx[3], dx[4], dx[5]});
-        V3 dx = p - ld3(w.pos0[h]);
-        V3 dr = quat_diff_vec(q, ldq(w.rot0[h]));
+    if (solve_6x6_div(s, dx)) {
+        V3 p = ld3(b.pos) + V3{dx[0], dx[1], dx[2]};
+        Q q = quat_integrate(ldq(b.rot), V3{dx[3], dx[4], dx[5]});
+        V3 d = p - ld3(b.pos0);
+        V3 dr = quat_diff_vec(q, ldq(b.rot0));
         w.pos[h] = st3(p, 0.0f);
         w.rot[h] = stq(q);
         float4* k = w.kin + (size_t)h * 4;
-        k[0] = st3(p, w.shp[h].x);
+        k[0] = st3(p, b.par);
         k[1] = stq(q);
-        k[2] = st3(dx, __uint_as_float(w.info[h]));
+        k[2] = st3(d, __uint_as_float(b.info));
         k[3] = st3(dr, 0.0f);
     } else {
         atomicAdd(&w.ctr[C_BREAKDOWN], 1u);  // breakdown: the body skips its update
     }
 }
 
-// One thread per body: rows accumulate in the reference's order (pairs in
-// ascending index — B-side pairs precede A-side ones — then joints).
 // JT: 0 for worlds without joints (the joint rows' code and registers stay
 // out of the contact-only kernels), 1 with ball and revolute joints only,
 // 2 with any joint kind.
-template <int MINB, int JT>
-__global__ void __launch_bounds__(128, MINB) k_primal_thread(DW w, int colour) {
-    if (aborted_solve(w)) return;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t c0 = w.col_cnt[colour], c1 = w.col_cnt[colour + 1];
-    if (c0 + i >= c1) return;
-    uint32_t h = w.col_list[c0 + i];
-    Sys s;
-    inertial_block(w, h, s);
-    for (uint32_t k = w.offB[h]; k < w.offB[h + 1]; k++) {
-        uint32_t p = w.listB[k];
-        PairCtx c;
-        load_ctx(w, p, c);
-        for (uint32_t q = 0; q < c.np; q++) stamp_point(w, c, p, q, false, s);
-    }
-    for (uint32_t p = w.offA[h]; p < w.offA[h + 1]; p++) {
-        PairCtx c;
-        load_ctx(w, p, c);
-        for (uint32_t q = 0; q < c.np; q++) stamp_point(w, c, p, q, true, s);
-    }
-    if (JT)
-        for (uint32_t k = w.jofs[h]; k < w.jofs[h + 1]; k++) stamp_joint<JT == 2>(w, w.jlist[k], h, s);
-    apply_solve(w, h, s);
-}
 
 // L lanes per body: the body's incident pairs are dealt round-robin over the
 // lanes, the partial systems are summed with shuffles, lane 0 adds the
@@ -504,27 +574,17 @@ __global__ void k_primal_lanes(DW w, int colour) {
     }
     if (!active || lane != 0) return;
     Sys t;
-    inertial_block(w, h, t);
+    inertial_block(w, h, recip_dt2(w), t);
 #pragma unroll
     for (int k = 0; k < 21; k++) t.h[k] += s.h[k];
 #pragma unroll
     for (int k = 0; k < 6; k++) t.r[k] += s.r[k];
     if (JT)
         for (uint32_t k = w.jofs[h]; k < w.jofs[h + 1]; k++) stamp_joint<JT == 2>(w, w.jlist[k], h, t);
-    apply_solve(w, h, t);
+    apply_solve(w, h, load_pose(w, h), t);
 }
 
-// ---- split primal -------------------------------------------------------------------
-// Per colour, phase 1 (k_side_rows) computes for every (pair, side) whose body
-// has this colour the pair's rows for that body, summed over its points, and
-// stores the 27 numbers in the incidence slot of that body; phase 2
-// (k_side_solve) gives each body of the colour its inertial block plus its
-// slots in incidence order (B-side pairs ascending, then A-side pairs
-// ascending), then its joints, and solves.  Phase 1 has one thread per
-// (pair, side) instead of one per body: several times more threads and short
-// dependency chains, which is what the latency-bound per-body loop lacks once
-// bodies touch many others.  Rows are summed per pair before they join the
-// body's sum, so results equal the thread-per-body kernel's within rounding.
+// ---- per-colour (pair, side) lists: what the reverse sweep's row kernel walks ------
 // Slots: body h owns [offA[h] + offB[h], offA[h+1] + offB[h+1]), B sides first;
 // the A side of pair p is slot p + offB[a+1], the B side slot offA[b] + posB[p].
 constexpr int SIDE_BLOCK = 256;
@@ -587,34 +647,6 @@ __global__ void k_side_place(DW w) {
     }
 }
 
-// The rows of pair p for its body on side side_a, summed over the pair's
-// points in point order: 21 Hessian + 6 rhs numbers as 7 float4 at o.
-static __device__ __forceinline__ void side_rows(const DW& w, uint32_t p, bool side_a, PairCtx& c, float4* o) {
-    Sys s;
-#pragma unroll
-    for (int k = 0; k < 21; k++) s.h[k] = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 6; k++) s.r[k] = 0.0f;
-    for (uint32_t q = 0; q < c.np; q++) stamp_point(w, c, p, q, side_a, s);
-    o[0] = make_float4(s.h[0], s.h[1], s.h[2], s.h[3]);
-    o[1] = make_float4(s.h[4], s.h[5], s.h[6], s.h[7]);
-    o[2] = make_float4(s.h[8], s.h[9], s.h[10], s.h[11]);
-    o[3] = make_float4(s.h[12], s.h[13], s.h[14], s.h[15]);
-    o[4] = make_float4(s.h[16], s.h[17], s.h[18], s.h[19]);
-    o[5] = make_float4(s.h[20], s.r[0], s.r[1], s.r[2]);
-    o[6] = make_float4(s.r[3], s.r[4], s.r[5], 0.0f);
-}
-// Add one incidence slot's 7 float4 to a body's system (k_side_solve's order).
-static __device__ __forceinline__ void add_slot(Sys& s, const float4* o) {
-    float4 v0 = o[0], v1 = o[1], v2 = o[2], v3 = o[3], v4 = o[4], v5 = o[5], v6 = o[6];
-    s.h[0] += v0.x; s.h[1] += v0.y; s.h[2] += v0.z; s.h[3] += v0.w;
-    s.h[4] += v1.x; s.h[5] += v1.y; s.h[6] += v1.z; s.h[7] += v1.w;
-    s.h[8] += v2.x; s.h[9] += v2.y; s.h[10] += v2.z; s.h[11] += v2.w;
-    s.h[12] += v3.x; s.h[13] += v3.y; s.h[14] += v3.z; s.h[15] += v3.w;
-    s.h[16] += v4.x; s.h[17] += v4.y; s.h[18] += v4.z; s.h[19] += v4.w;
-    s.h[20] += v5.x; s.r[0] += v5.y; s.r[1] += v5.z; s.r[2] += v5.w;
-    s.r[3] += v6.x; s.r[4] += v6.y; s.r[5] += v6.z;
-}
 // Work lists are taken in chunks of one block (128 entries) whose entries are
 // handed to the block's threads grouped by a small work class (the entry's
 // loop length), so that the lanes of a warp run loops of the same length
@@ -643,94 +675,58 @@ static __device__ __forceinline__ uint32_t chunk_sort(uint32_t* cnt, uint32_t* e
     __syncthreads();
     return n;
 }
-__global__ void __launch_bounds__(CHUNK, 4) k_side_rows(DW w, int colour) {
-    if (aborted_solve(w)) return;
-    __shared__ uint32_t s_cnt[MAX_PTS + 1], s_ent[CHUNK];
-    const uint32_t s0 = w.side_cnt[colour], s1 = w.side_cnt[colour + 1];
-    for (uint32_t base = s0 + blockIdx.x * CHUNK; base < s1; base += gridDim.x * CHUNK) {
-        const uint32_t i = base + threadIdx.x;
-        const bool has = i < s1;
-        uint32_t e = 0, cls = 0;
-        if (has) {
-            e = w.side_list[i];
-            uint32_t p = e >> 1;
-            cls = w.p_n[p].w <= 0.0f ? w.p_np[p] : 0u;  // separated pairs stamp at most a damper row
-        }
-        const uint32_t n = chunk_sort(s_cnt, s_ent, has, e, cls, min((uint32_t)CHUNK, s1 - base));
-        if (threadIdx.x < n) {
-            e = s_ent[threadIdx.x];
-            uint32_t p = e >> 1;
-            bool side_a = (e & 1u) != 0u;
-            PairCtx c;
-            load_ctx(w, p, c);
-            uint32_t slot = side_a ? p + w.offB[c.a + 1] : w.offA[c.b] + w.posB[p];
-            // a recording frame too small: the host reports it
-            if (slot < w.contrib_slots) side_rows(w, p, side_a, c, w.contrib + (size_t)slot * 7);
-        }
-        __syncthreads();  // the chunk's entries are read before the next chunk is sorted
-    }
-}
-template <int JT>
-__global__ void __launch_bounds__(128) k_side_solve(DW w, int colour) {
-    if (aborted_solve(w)) return;
-    const uint32_t c0 = w.col_cnt[colour], c1 = w.col_cnt[colour + 1];
-    for (uint32_t i = c0 + blockIdx.x * blockDim.x + threadIdx.x; i < c1; i += gridDim.x * blockDim.x) {
-        uint32_t h = w.col_list[i];
-        Sys s;
-        inertial_block(w, h, s);
-        const uint32_t k0 = w.offA[h] + w.offB[h], k1 = min(w.offA[h + 1] + w.offB[h + 1], w.contrib_slots);
-        for (uint32_t k = k0; k < k1; k++) add_slot(s, w.contrib + (size_t)k * 7);
-        if (JT)
-            for (uint32_t k = w.jofs[h]; k < w.jofs[h + 1]; k++) stamp_joint<JT == 2>(w, w.jlist[k], h, s);
-        apply_solve(w, h, s);
-    }
-}
-
-// ---- dual (joints_ext.rs:464-573 contacts, :574-896 Ball/Revolute) ----
-// One thread per pair: the pair context is built once for all its points.
-static __device__ __forceinline__ void dual_point(const DW& w, const PairCtx& c, V3 t1, V3 t2, uint32_t q) {
-    float4 ra = w.q_ra[q], rb = w.q_rb[q];
-    bool touching = c.gap <= 0.0f;
-    float4 pen = w.q_pen[q], lam = w.q_lam[q];
-    float c0 = touching ? lam.w : 0.0f;
-    V3 raw, rbw;
-    contact_levers(c, ra, rb, raw, rbw);
-    float cn = row_c_levers(c, c.n, c0, raw, rbw);
-    V3 raf, rbf;
-    friction_levers(c, raw, rbw, raf, rbf);
-    float ct1 = row_c_levers(c, t1, 0.0f, raf, rbf);
-    float ct2 = row_c_levers(c, t2, 0.0f, raf, rbf);
+// ---- dual (joints_ext.rs:464-573 contacts, :574-896 joints) ----
+// The dual update of a point from its constraint values: its new multipliers
+// and penalties into lam and pen, stored with the grip flag (rbw: the flag as
+// stored).
+static __device__ __forceinline__ void dual_update(const DW& w, const PairCtx& c, const ContactGeo& g, uint32_t q, float rbw,
+                                                   float4& lam, float4& pen) {
+    const bool touching = c.gap <= 0.0f;
     float f[3];
-    contact_force(cn, pen, lam, ct1, ct2, c.mu, f);
+    contact_force(g.cn, pen, lam, g.ct1, g.ct2, c.mu, f);
     float bnd = fabsf(f[0]) * fmaxf(c.mu.x, c.mu.y);
-    float fu0 = pen.y * ct1 + lam.y, fu1 = pen.z * ct2 + lam.z;
-    bool stuck = sqrtf(fu0 * fu0 + fu1 * fu1) <= bnd && sqrtf(ct1 * ct1 + ct2 * ct2) < STICK_THRESH;
+    float fu0 = pen.y * g.ct1 + lam.y, fu1 = pen.z * g.ct2 + lam.z;
+    bool stuck = sqrt0(fu0 * fu0 + fu1 * fu1) <= bnd && sqrt0(g.ct1 * g.ct1 + g.ct2 * g.ct2) < STICK_THRESH;
     float4 nl = lam, np4 = pen;
-    if (touching && fabsf(cn) >= C_EPS) {
+    if (touching && fabsf(g.cn) >= C_EPS) {
         nl.x = f[0];
-        if (f[0] < 0.0f) np4.x = fminf(pen.x + BETA * fabsf(cn), PENALTY_MAX);
+        if (f[0] < 0.0f) np4.x = fminf(pen.x + BETA * fabsf(g.cn), PENALTY_MAX);
     }
     float b1 = fabsf(f[0]) * c.mu.x, b2 = fabsf(f[0]) * c.mu.y;
-    float s_ell = (b1 > 0.0f && b2 > 0.0f) ? (fu0 / b1) * (fu0 / b1) + (fu1 / b2) * (fu1 / b2) : INFINITY;
+    float s_ell = INFINITY;
+    if (b1 > 0.0f && b2 > 0.0f) {
+        const float g0 = div0(fu0, b1), g1 = div0(fu1, b2);
+        s_ell = g0 * g0 + g1 * g1;
+    }
     if (touching) {
         nl.y = f[1];
         nl.z = f[2];
         if (s_ell <= 1.0f) {
-            if (fabsf(ct1) >= C_EPS) np4.y = fminf(pen.y + BETA * fabsf(ct1), PENALTY_MAX);
-            if (fabsf(ct2) >= C_EPS) np4.z = fminf(pen.z + BETA * fabsf(ct2), PENALTY_MAX);
+            if (fabsf(g.ct1) >= C_EPS) np4.y = fminf(pen.y + BETA * fabsf(g.ct1), PENALTY_MAX);
+            if (fabsf(g.ct2) >= C_EPS) np4.z = fminf(pen.z + BETA * fabsf(g.ct2), PENALTY_MAX);
         }
     }
     w.q_lam[q] = nl;
     // penalties and the grip flag change in few iterations: store only changes
     if (np4.x != pen.x || np4.y != pen.y || np4.z != pen.z) w.q_pen[q] = np4;
-    if (stuck != (rb.w != 0.0f)) reinterpret_cast<float*>(&w.q_rb[q])[3] = stuck ? 1.0f : 0.0f;
+    if (stuck != (rbw != 0.0f)) reinterpret_cast<float*>(&w.q_rb[q])[3] = stuck ? 1.0f : 0.0f;
+    lam = nl;
+    pen = np4;
+}
+static __device__ __forceinline__ void dual_point(const DW& w, const PairCtx& c, uint32_t q, float4& lam, float4& pen) {
+    const bool touching = c.gap <= 0.0f;
+    const float4 rb = w.q_rb[q];
+    lam = w.q_lam[q];
+    pen = w.q_pen[q];
+    const ContactGeo g = contact_geo(c, w.q_ra[q], rb, touching ? lam.w : 0.0f, true);
+    dual_update(w, c, g, q, rb.w, lam, pen);
     const float mu_roll = c.mu_roll, mu_spin = c.mu_spin;
     if (touching && (mu_roll > 0.0f || mu_spin > 0.0f)) {
         V3 wrel = c.dra - c.drb;
-        float lam_n = fabsf(nl.x);
+        float lam_n = fabsf(lam.x);
         float4 rl = w.q_roll[q];
         float rls[3] = {rl.x, rl.y, rl.z};
-        V3 rax[3] = {t1, t2, c.n};
+        V3 rax[3] = {c.t1, c.t2, c.n};
         float murs[3] = {mu_roll, mu_roll, mu_spin};
         for (int li = 0; li < 3; li++) {
             if (murs[li] <= 0.0f) continue;
@@ -745,9 +741,8 @@ static __device__ __forceinline__ void dual_pair(const DW& w, uint32_t p) {
     if (np == 0) return;
     PairCtx c;
     load_ctx(w, p, c);
-    V3 t1 = tangent_t1(c.n);  // the grip flag of separated points needs the frame too
-    V3 t2 = cross(t1, c.n);
-    for (uint32_t k = 0; k < np; k++) dual_point(w, c, t1, t2, p * MAX_PTS + k);
+    float4 lam, pen;
+    for (uint32_t k = 0; k < np; k++) dual_point(w, c, p * MAX_PTS + k, lam, pen);
 }
 __global__ void __launch_bounds__(CHUNK) k_dual_pairs(DW w) {
     if (aborted_solve(w)) return;
@@ -1020,234 +1015,641 @@ __global__ void k_dual_joints(DW w) {
     if (j < (uint32_t)w.J) dual_joint<ALL>(w, j);
 }
 
-// ---- per-scene solve: one block walks a scene through every iteration ---------
-// Scenes never interact, so a block can take one scene through all
-// iterations of a substep — every colour's primal, then the scene's dual —
-// with block barriers between the phases and no wait on any other block.
-// The scene's data (its bodies' motion records, pairs and points) is touched
-// iterations x (colours + 1) times within one block, so after the first
-// touch it is served from L2 instead of being streamed from HBM once per
-// launch.  Blocks take scenes from a queue in descending size order (the
-// longest first), so the largest scenes do not finish last.
+// ---- tile engine: every iteration of a substep in one launch --------------------
+// A body's system is the inertial block plus its rows in incidence order
+// (B-side pairs ascending, then A-side pairs ascending, their points in
+// order, then its joints).  One thread per body pays a dependent chain of
+// loads and about 600 instructions per point (46 us a colour for 35 cubes of
+// 20 points each); one thread per (pair, side) writes and re-reads 112 bytes
+// per incidence.  Here a warp takes up to 32 bodies of one colour and splits
+// the work by what is independent:
+//   rows   one lane per (point, side) or third of a joint computes its rows
+//          into the warp's shared memory, 32 at a time;
+//   sums   27 lanes, each owning one number of the 6x6 system, add the rows in
+//          their order: the same additions in the same order as one thread
+//          would make, so the sum is bit-identical;
+//   solve  one lane per body factors and applies.
+// Warps share nothing between barriers, so the latency of one (a chain of
+// loads, then divisions and square roots) is covered by the others; bodies
+// are dealt to as many warps as there are, 32 to a warp only once every warp
+// has some.
+// PS = false sums row by row (the thread-per-body order, the reference's);
+// PS = true sums each pair's rows from zero first and adds the pair's sum
+// (the split order).
 //
-// Arithmetic is the split primal's: per (pair, side) the pair's rows summed
-// over its points (one thread per item, staged in shared memory), then per
-// body the inertial block, its items in incidence order and its joints, and
-// the 6x6 solve (one owner thread per body); the dual per pair and per joint.
-// Bodies of one colour share no pair or joint, so the order in which a
-// colour's bodies are visited cannot change a result.
+// Bound by latency, not by bytes: a colour costs a lone warp about 2 us of
+// item rows, 0.6 us of sums, 1.7 us of solves and 1 us of barrier; with every
+// warp busy (100,000 bodies) the schedulers issue 40% of their slots.
+// Iterations of a substep, before (a launch per colour) and after, in ms:
+// 210-cube pyramid 3.25 -> 0.55, 1500-body heap 1.60 -> 0.27, 96 scenes of up
+// to 400 bodies 1.44 -> 0.25, 1536 scenes of up to 1024 bodies 3.02 -> 2.42,
+// 100,000 bodies on a plane 2.03 -> 1.07, 1200 ragdolls 2.37 -> 1.28.  A
+// cluster per scene (its own barriers) was slower at every size but one
+// (0.34, 0.33 and 3.1 ms for the heap and the two batches): warps idle at
+// their own scene's barriers.
+//
+// k_entries lists, once per substep, every body's (point, side) items, so
+// that an item's lane goes straight to its data.  The list lives in the
+// previous generation's point anchors (q_ra, q_rb), which nothing reads once
+// discovery has merged them.
 
-// In-place exclusive scan of a[0..n) (n <= SCENE_MAX_BODIES) by the block;
-// a[n] receives the total.  Needs 32 words of scratch.
-template <int BS>
-static __device__ __forceinline__ void block_scan(uint32_t* a, uint32_t n, uint32_t* warp_tot) {
-    const uint32_t per = (n + BS - 1) / BS;
-    const uint32_t t = threadIdx.x, i0 = min(n, t * per), i1 = min(n, i0 + per);
-    uint32_t sum = 0;
-    for (uint32_t i = i0; i < i1; i++) sum += a[i];
-    const uint32_t lane = t & 31u, wid = t >> 5;
-    uint32_t inc = sum;
+constexpr uint32_t ENT_SIDE_A = 1u << 31;  // the body is the pair's A side
+constexpr uint32_t ENT_LAST = 1u << 30;    // last item of its pair
+constexpr uint32_t ENT_ROLL = 1u << 29;    // the point's rolling and torsion rows
+constexpr uint32_t ENT_DUAL = 1u << 28;    // this side updates the point's dual (the pair's first swept colour)
+constexpr uint32_t ENT_BODY = ENT_DUAL - 1u;  // the other body
+constexpr uint32_t ENT_PER_SLOT = 2 * MAX_PTS;  // items of one incidence slot: 8 points, twice with rolling
+
+// Eight lanes per body walk its incidence slots; einfo[h] = (first slot, items).
+__global__ void __launch_bounds__(256) k_entries(DW w) {
+    if (aborted_solve(w)) return;
+    const uint32_t h = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, l8 = threadIdx.x & 7u;
+    if (h >= (uint32_t)w.N || w.colour[h] < 0) return;
+    const uint32_t mask = 0xffu << (threadIdx.x & 24u);
+    const uint32_t a0 = w.offA[h], b0 = w.offB[h], nB = w.offB[h + 1] - b0, n = nB + w.offA[h + 1] - a0;
+    uint2* out = w.ent + (size_t)(a0 + b0) * ENT_PER_SLOT;
+    uint32_t cnt = 0;
+    for (uint32_t j0 = 0; j0 < n; j0 += 8) {
+        const uint32_t j = j0 + l8;
+        const bool side_a = j >= nB;
+        uint32_t p = 0, np = 0, other = 0;
+        bool roll = false, dual = false;
+        if (j < n) {
+            p = side_a ? a0 + (j - nB) : w.listB[b0 + j];
+            np = min(w.p_np[p], (uint32_t)MAX_PTS);
+            const uint2 ab = w.p_ab[p];
+            other = side_a ? ab.y : ab.x;
+            const int co = w.colour[other];
+            dual = co < 0 || w.colour[h] < co;
+            if (w.p_n[p].w <= 0.0f) {
+                const float4 ma = w.mat[ab.x], mb = w.mat[ab.y];
+                roll = fmaxf(ma.z, mb.z) > 0.0f || fmaxf(ma.w, mb.w) > 0.0f;
+            }
+        }
+        const uint32_t m = roll ? 2u * np : np;
+        uint32_t inc = m;
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(mask, inc, o, 8);
+            if (l8 >= (uint32_t)o) inc += v;
+        }
+        uint2* e = out + cnt + (inc - m);
+        if (roll && np) w.ctr[C_ROLL] = 1u;
+        const uint32_t tag = other | (side_a ? ENT_SIDE_A : 0u) | (dual ? ENT_DUAL : 0u);
+        for (uint32_t k = 0; k < np; k++) {
+            const uint32_t last = k + 1 == np ? ENT_LAST : 0u;
+            *e++ = make_uint2(p * MAX_PTS + k, tag | (roll ? 0u : last));
+            if (roll) *e++ = make_uint2(p * MAX_PTS + k, tag | ENT_ROLL | last);
+        }
+        cnt += __shfl_sync(mask, inc, 7, 8);
+    }
+    if (l8 == 0) w.einfo[h] = make_uint2(a0 + b0, cnt);
+}
+
+constexpr int SLOT = 36;        // floats of an item's slot: 8 float4, padded so that 32 slots spread over the banks
+constexpr int SYS_STRIDE = 27;  // 21 Hessian + 6 right-hand-side numbers (odd: no bank conflicts)
+constexpr uint32_t JOINT_PARTS = 3;  // items of a joint: up to 9 rows (revolute with a limit: 7)
+// an item's control word: row types (6 bits), last item of its pair, a joint's
+constexpr uint32_t CTL_LAST = 1u << 8, CTL_JOINT = 1u << 9;
+constexpr uint32_t CTL_MIXED = 1u << 10;  // a row that is not ROW_FULL
+
+struct WarpMem {
+    float rows[35 * SLOT];  // the sums read up to three slots past the last
+    float sys[32 * SYS_STRIDE];
+    float ones[4];
+};
+
+// The number of the 6x6 system a lane owns, as float offsets into a slot:
+// value += slot[c] * (slot[a] * slot[b]).
+struct Elem {
+    int a, b, c;
+    int own;              // the number's index (a lane past 26 repeats 26)
+    bool rhs, ang, diag;  // right-hand side; both factors angular; an angular diagonal
+};
+static __device__ __forceinline__ Elem elem_of(int lane) {
+    Elem e;
+    e.own = lane < SYS_STRIDE ? lane : SYS_STRIDE - 1;
+    int i = 0, j = 0;
+    e.rhs = lane >= 21;
+    if (e.rhs) {
+        i = lane < 27 ? lane - 21 : 0;
+    } else {
+        while (lane >= tri(i + 1, 0)) i++;
+        j = lane - tri(i, 0);
+    }
+    e.a = 4 * (i < 3 ? i : i + 1);
+    e.b = 4 * (j < 3 ? j : j + 1);
+    e.c = e.rhs ? 28 : 12;
+    e.ang = i >= 3 && (e.rhs || j >= 3);
+    e.diag = !e.rhs && i >= 3 && i == j;
+    return e;
+}
+// A lane's terms of a slot's three rows (dg: the value a diagonal row adds).
+struct Terms {
+    float x, y, z;
+    float dx, dy, dz;
+};
+static __device__ __forceinline__ Terms slot_terms(const float* slot, const float* ones, const Elem& e) {
+    const float4 A = *reinterpret_cast<const float4*>(slot + e.a);
+    const float4 B = *reinterpret_cast<const float4*>(e.rhs ? ones : slot + e.b);
+    const float4 C = *reinterpret_cast<const float4*>(slot + e.c);
+    return Terms{C.x * (A.x * B.x), C.y * (A.y * B.y), C.z * (A.z * B.z), A.x, A.y, A.z};
+}
+static __device__ __forceinline__ void add_row(float& s, uint32_t type, float v, float diag, const Elem& e) {
+    if (type == ROW_FULL || (type == ROW_ANG && e.ang)) s += v;
+    else if (type == ROW_DIAG && e.diag) s += diag;
+}
+// Add a slot's rows, in order, to the lane's number.
+static __device__ __forceinline__ void add_terms(const Terms& t, uint32_t ctl, const Elem& e, float& s) {
+    add_row(s, ctl & 3u, t.x, t.dx, e);
+    add_row(s, (ctl >> 2) & 3u, t.y, t.dy, e);
+    add_row(s, (ctl >> 4) & 3u, t.z, t.dz, e);
+}
+
+// What a recording rollout keeps: a point's state after the dual of iteration
+// slice - 1, a body's pose after the sweep of it (slice 0 is the start).
+static __device__ __forceinline__ void record_point(const IterRec& rec, int slice, uint32_t q, float4 lam, float4 pen) {
+    if (q >= rec.qcap) return;  // a frame too small: the host reports it
+    rec.lam[(size_t)slice * rec.qstride + q] = lam;
+    rec.pen[(size_t)slice * rec.qstride + q] = pen;
+}
+static __device__ __forceinline__ void record_pose(const DW& w, const IterRec& rec, int slice, uint32_t h) {
+    const size_t i = (size_t)slice * (size_t)w.N + h;
+    rec.pos[i] = w.pos[h];
+    rec.rot[i] = w.rot[h];
+}
+// One iteration of the engine: whether this iteration's items first update
+// their points' duals (of the iteration before), and what is recorded.
+struct IterCtx {
+    int it;
+    bool dual;
+    float* contrib;  // null, or recording: where the pairs' sums go, 28 floats per incidence slot
+};
+// the sum of the pair whose last item holds `slot`
+static __device__ __forceinline__ void keep_pair(const IterRec& rec, const IterCtx& ic, const float* slot, float ps) {
+    const uint32_t lane = threadIdx.x & 31u, q = __float_as_uint(slot[SLOT - 1]);
+    if (lane < SYS_STRIDE && q < rec.slots) ic.contrib[(size_t)q * 28 + lane] = ps;  // else the host reports it
+}
+// An item of body h: a (point, side) of its list, or a third of joint e.x.
+struct Item {
+    uint32_t h;
+    uint2 e;
+    bool joint;
+};
+// The item's rows into the lane's slot; returns its control word.
+template <int JT, bool PS, bool REC>
+static __device__ __forceinline__ uint32_t item_rows(const DW& w, const IterRec& rec, const IterCtx& ic, float* slot,
+                                                     const Item& im) {
+    const uint32_t h = im.h;
+    const uint2 e = im.e;
+    if (JT && im.joint) {
+        RowSink sink{slot, (int)(3u * e.y), 0, 0u};
+        stamp_joint<JT == 2>(w, e.x, h, sink);
+        return sink.types | CTL_JOINT | CTL_MIXED;
+    }
+    const bool side_a = (e.y & ENT_SIDE_A) != 0u, dual = ic.dual && (e.y & ENT_DUAL);
+    const uint32_t other = e.y & ENT_BODY, p = e.x / MAX_PTS;
+    const float4 ra = w.q_ra[e.x], rb = w.q_rb[e.x];
+    float4 lam = w.q_lam[e.x], pen = w.q_pen[e.x];
+    PairCtx c;
+    load_ctx(w, p, side_a ? make_uint2(h, other) : make_uint2(other, h), c);
+    const bool touching = c.gap <= 0.0f;
+    const ContactGeo g = contact_geo(c, ra, rb, touching ? lam.w : 0.0f, touching || dual);
+    if (dual) {
+        dual_update(w, c, g, e.x, rb.w, lam, pen);
+        if (REC && ic.contrib) record_point(rec, ic.it, e.x, lam, pen);
+    }
+    const ContactRows r = contact_rows(w, c, g, side_a, lam, pen);
+    uint32_t ctl = (e.y & ENT_LAST) ? CTL_LAST : 0u;
+    if (e.y & ENT_ROLL) {
+        load_rolling(w, c);
+        RowSink sink{slot, 0, 0, 0u};
+        stamp_rolling(w, c, e.x, side_a, r.f[0], sink);
+        ctl |= sink.types | CTL_MIXED;
+    } else {
+        const float sign = side_a ? 1.0f : -1.0f;
+        const V3 n0 = sign * c.n, n1 = sign * c.t1, n2 = sign * c.t2;
+        const V3 m0 = cross(r.lever, n0), m1 = cross(r.lever_f, n1), m2 = cross(r.lever_f, n2);
+        float4* o = reinterpret_cast<float4*>(slot);
+        o[0] = make_float4(n0.x, n1.x, n2.x, 0.0f);
+        o[1] = make_float4(n0.y, n1.y, n2.y, 0.0f);
+        o[2] = make_float4(n0.z, n1.z, n2.z, 0.0f);
+        o[3] = make_float4(r.pen[0], r.pen[1], r.pen[2], 0.0f);
+        o[4] = make_float4(m0.x, m1.x, m2.x, 0.0f);
+        o[5] = make_float4(m0.y, m1.y, m2.y, 0.0f);
+        o[6] = make_float4(m0.z, m1.z, m2.z, 0.0f);
+        o[7] = make_float4(r.f[0], r.f[1], r.f[2], 0.0f);
+        ctl |= (r.live & 1u) | (r.live & 2u) << 1 | (r.live & 4u) << 2;
+    }
+    if (REC && ic.contrib && (ctl & CTL_LAST))  // the pair's incidence slot, in the slot's padding
+        slot[SLOT - 1] = __uint_as_float(side_a ? p + w.offB[h + 1] : w.offA[h] + w.posB[p]);
+    return ctl;
+}
+
+// A warp's tile, bodies list[i0 .. i0 + nb) of one colour (nb <= 32): lane i
+// holds body i's item count and its first item among the tile's `total`.
+struct Tile {
+    uint32_t nb, total;
+    uint32_t h, first, ne, cnt, pre, j0;
+    Item im;  // the lane's item of the first round
+};
+// The lane's item g of the tile (fetch: also its list entry), its body's lane.
+template <int JT>
+static __device__ __forceinline__ Item tile_item(const DW& w, const Tile& t, uint32_t g, uint32_t& b, bool fetch) {
+    const uint32_t all = 0xffffffffu;
+    // its body: the last lane whose first item is at or before it
+    b = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1) {
+        const uint32_t v = __shfl_sync(all, t.pre, b + step);
+        if (v <= g) b += step;
+    }
+    const uint32_t h = __shfl_sync(all, t.h, b), first = __shfl_sync(all, t.first, b), ne = __shfl_sync(all, t.ne, b);
+    const uint32_t k = g - __shfl_sync(all, t.pre, b), j0 = JT ? __shfl_sync(all, t.j0, b) : 0u;
+    Item im{h, make_uint2(0u, 0u), false};
+    if (g < t.total) {
+        if (JT && k >= ne) {
+            im.joint = true;
+            if (fetch) im.e = make_uint2(w.jlist[j0 + (k - ne) / JOINT_PARTS], (k - ne) % JOINT_PARTS);
+        } else if (fetch) {
+            im.e = w.ent[(size_t)first * ENT_PER_SLOT + k];
+        }
+    }
+    return im;
+}
+// What a tile needs that no other body's move changes: its items and its
+// bodies' inertial blocks (a body's own pose moves only in its own solve).
+// Run while a barrier is being waited for.
+template <int JT>
+static __device__ __forceinline__ Tile open_tile(const DW& w, WarpMem& sm, const Recip& rdt2, const uint32_t* list,
+                                                 uint32_t i0, uint32_t nb) {
+    const uint32_t lane = threadIdx.x & 31u, all = 0xffffffffu;
+    Tile t{nb, 0, 0, 0, 0, 0, 0, 0, Item{0, make_uint2(0u, 0u), false}};
+    if (nb == 0) return t;
+    uint32_t nj = 0;
+    if (lane < nb) {
+        t.h = list[i0 + lane];
+        const uint2 ei = w.einfo[t.h];
+        t.first = ei.x;
+        t.ne = ei.y;
+        if (JT) {
+            t.j0 = w.jofs[t.h];
+            nj = w.jofs[t.h + 1] - t.j0;
+        }
+    }
+    t.cnt = t.ne + JOINT_PARTS * nj;
+    uint32_t pre = t.cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= (uint32_t)o) inc += v;
+        const uint32_t v = __shfl_up_sync(all, pre, o);
+        if (lane >= (uint32_t)o) pre += v;
     }
-    if (lane == 31) warp_tot[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-        uint32_t v = lane < BS / 32 ? warp_tot[lane] : 0u, x = v;
+    t.total = __shfl_sync(all, pre, 31);
+    t.pre = pre - t.cnt;  // past the last body: total
+    uint32_t b;
+    t.im = tile_item<JT>(w, t, lane, b, true);
+    if (lane < nb) {
+        Sys s;
+        inertial_block(w, t.h, rdt2, s);
+        float* o = sm.sys + lane * SYS_STRIDE;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= (uint32_t)o) x += y;
-        }
-        if (lane < BS / 32) warp_tot[lane] = x - v;  // exclusive warp offsets
-        if (lane == BS / 32 - 1) a[n] = x;          // the total (a[n] is past every thread's chunk)
+        for (int k = 0; k < 21; k++) o[k] = s.h[k];
+#pragma unroll
+        for (int k = 0; k < 6; k++) o[21 + k] = s.r[k];
     }
-    __syncthreads();
-    uint32_t run = warp_tot[wid] + inc - sum;
-    for (uint32_t i = i0; i < i1; i++) {
-        uint32_t v = a[i];
-        a[i] = run;
-        run += v;
-    }
-    __syncthreads();
+    return t;
 }
-
-template <int BS, int MINB, int JT>
-__global__ void __launch_bounds__(BS, MINB) k_scene_solve(DW w) {
-    if (aborted_solve(w)) return;
-    __shared__ uint32_t s_list[SCENE_MAX_BODIES];      // swept bodies grouped by colour
-    __shared__ uint32_t s_pref[SCENE_MAX_BODIES + 1];  // item offset of each list entry
-    __shared__ uint32_t s_cstart[MAX_COLOURS + 1];
-    __shared__ uint32_t s_cur[MAX_COLOURS];
-    __shared__ uint32_t s_warp[32];
-    __shared__ uint32_t s_scene;
-    __shared__ int s_ncol;
-    extern __shared__ float4 s_rows[];  // BS items x 7 float4
-    const uint32_t tid = threadIdx.x;
-    for (;;) {
-        if (tid == 0) s_scene = atomicAdd(&w.ctr[C_SCENE_Q], 1u);
-        __syncthreads();
-        const uint32_t q = s_scene;
-        if (q >= (uint32_t)w.S) return;
-        const uint32_t sc = w.scene_order[q];
-        const uint32_t b0 = w.scene_off[sc], b1 = w.scene_off[sc + 1];
-        // colour lists of the scene's swept bodies
-        for (uint32_t c = tid; c < MAX_COLOURS; c += BS) s_cur[c] = 0;
-        if (tid == 0) s_ncol = 0;
-        __syncthreads();
-        for (uint32_t h = b0 + tid; h < b1; h += BS) {
-            int c = w.colour[h];
-            if (c >= 0 && c < MAX_COLOURS) {
-                atomicAdd(&s_cur[c], 1u);
-                atomicMax(&s_ncol, c + 1);
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            uint32_t acc = 0;
-            for (int c = 0; c < s_ncol; c++) {
-                s_cstart[c] = acc;
-                acc += s_cur[c];
-                s_cur[c] = s_cstart[c];
-            }
-            s_cstart[s_ncol] = acc;
-        }
-        __syncthreads();
-        const int ncol = s_ncol;
-        const uint32_t nlist = s_cstart[ncol];
-        for (uint32_t h = b0 + tid; h < b1; h += BS) {
-            int c = w.colour[h];
-            if (c >= 0 && c < MAX_COLOURS) s_list[atomicAdd(&s_cur[c], 1u)] = h;
-        }
-        __syncthreads();
-        for (uint32_t i = tid; i < nlist; i += BS) {
-            uint32_t h = s_list[i];
-            s_pref[i] = (w.offA[h + 1] - w.offA[h]) + (w.offB[h + 1] - w.offB[h]);
-        }
-        __syncthreads();
-        block_scan<BS>(s_pref, nlist, s_warp);
-        const uint32_t p0 = w.offA[b0], p1 = w.offA[b1];
-        for (int it = 0; it < w.iterations; it++) {
-            for (int c = 0; c < ncol; c++) {
-                const uint32_t hi = s_cstart[c + 1];
-                for (uint32_t i0 = s_cstart[c]; i0 < hi;) {
-                    // a group: the next (up to) BS bodies of the colour, one
-                    // owner thread each; their items are computed BS per round
-                    const uint32_t base = s_pref[i0];
-                    const uint32_t i1 = min(hi, i0 + BS);
-                    const uint32_t nb = i1 - i0, nitems = s_pref[i1] - base;
-                    Sys s;
-                    uint32_t h = 0, my0 = 0, my1 = 0;
-                    if (tid < nb) {
-                        h = s_list[i0 + tid];
-                        inertial_block(w, h, s);
-                        my0 = s_pref[i0 + tid] - base;
-                        my1 = s_pref[i0 + tid + 1] - base;
-                    }
-                    for (uint32_t r0 = 0; r0 < nitems; r0 += BS) {
-                        const uint32_t g = r0 + tid;
-                        if (g < nitems) {
-                            // the body of item g: the last entry starting at or before it
-                            int lo = (int)i0, up = (int)i1 - 1;
-                            while (lo < up) {
-                                int m = (lo + up + 1) >> 1;
-                                if (s_pref[m] - base <= g) lo = m;
-                                else up = m - 1;
-                            }
-                            const uint32_t hb = s_list[lo], k = g - (s_pref[lo] - base);
-                            const uint32_t nB = w.offB[hb + 1] - w.offB[hb];
-                            const bool side_a = k >= nB;
-                            const uint32_t p = side_a ? w.offA[hb] + (k - nB) : w.listB[w.offB[hb] + k];
-                            PairCtx cx;
-                            load_ctx(w, p, cx);
-                            side_rows(w, p, side_a, cx, s_rows + (size_t)tid * 7);
+// Solve a tile by its warp.  A caller whose next bodies read the moved poses
+// synchronises first.
+template <int JT, bool PS, bool REC>
+static __device__ __forceinline__ void solve_tile(const DW& w, const IterRec& rec, const IterCtx& ic, WarpMem& sm,
+                                                  const Elem& el, const Tile& tile) {
+    const uint32_t lane = threadIdx.x & 31u, all = 0xffffffffu;
+    const uint32_t h = tile.h, pre = tile.pre, cnt = tile.cnt, total = tile.total;
+    __syncwarp();
+    float ps = 0.0f;  // sum of the pair being added (a pair's items may span two rounds)
+    for (uint32_t r0 = 0; r0 < total; r0 += 32) {
+        const uint32_t g = r0 + lane;
+        uint32_t b;
+        Item im = tile_item<JT>(w, tile, g, b, r0 != 0);
+        if (r0 == 0) im.e = tile.im.e;
+        uint32_t ctl = 0;
+        if (g < total) ctl = item_rows<JT, PS, REC>(w, rec, ic, sm.rows + lane * SLOT, im);
+        __syncwarp();
+        // which items have each row live, end a pair, hold other rows than ROW_FULL
+        const uint32_t m0 = __ballot_sync(all, ctl & 1u), m1 = __ballot_sync(all, ctl & 4u), m2 = __ballot_sync(all, ctl & 16u);
+        const uint32_t ml = PS ? __ballot_sync(all, ctl & CTL_LAST) : 0u;
+        const bool plain = !__any_sync(all, ctl & CTL_MIXED);
+        const uint32_t n = min(32u, total - r0);
+        const uint32_t blast = __shfl_sync(all, b, n - 1);
+        for (uint32_t bb = __shfl_sync(all, b, 0); bb <= blast; bb++) {
+            const uint32_t f = __shfl_sync(all, pre, bb), e1 = min(f + __shfl_sync(all, cnt, bb), r0 + 32u) - r0;
+            const uint32_t e0 = max(f, r0) - r0;
+            if (f >= r0 + 32u || e0 >= e1) continue;
+            float s = sm.sys[bb * SYS_STRIDE + el.own];
+            if (plain) {
+                // four items a round: their loads and products are independent, the sums follow in
+                // order (bits past the body's last item are off)
+                const uint32_t own = e1 < 32u ? (1u << e1) - 1u : all;
+                const uint32_t x0 = m0 & own, x1 = m1 & own, x2 = m2 & own, xl = ml & own;
+                for (uint32_t e = e0; e < e1; e += 4) {
+                    Terms t[4];
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++) t[k] = slot_terms(sm.rows + (e + k) * SLOT, sm.ones, el);
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; k++) {
+                        float& acc = PS ? ps : s;
+                        if ((x0 >> e) & (1u << k)) acc += t[k].x;
+                        if ((x1 >> e) & (1u << k)) acc += t[k].y;
+                        if ((x2 >> e) & (1u << k)) acc += t[k].z;
+                        if (PS && ((xl >> e) & (1u << k))) {
+                            if (REC && ic.contrib) keep_pair(rec, ic, sm.rows + (e + k) * SLOT, ps);
+                            s += ps;
+                            ps = 0.0f;
                         }
-                        __syncthreads();
-                        if (tid < nb) {
-                            const uint32_t e1 = min(my1, r0 + BS);
-                            for (uint32_t e = max(my0, r0); e < e1; e++) add_slot(s, s_rows + (size_t)(e - r0) * 7);
-                        }
-                        __syncthreads();
                     }
-                    if (tid < nb) {
-                        if (JT)
-                            for (uint32_t k = w.jofs[h]; k < w.jofs[h + 1]; k++) stamp_joint<JT == 2>(w, w.jlist[k], h, s);
-                        apply_solve(w, h, s);
-                    }
-                    i0 = i1;
                 }
-                __syncthreads();  // this colour's poses before the next colour reads them
-            }
-            for (uint32_t p = p0 + tid; p < p1; p += BS) dual_pair(w, p);
-            if (JT)
-                for (uint32_t h = b0 + tid; h < b1; h += BS)
-                    for (uint32_t k = w.jofs[h]; k < w.jofs[h + 1]; k++) {
-                        uint32_t j = w.jlist[k];
-                        if (joint_dual_owner(w, j) == h) dual_joint<JT == 2>(w, j);
+            } else {
+                for (uint32_t e = e0; e < e1; e++) {
+                    const uint32_t c = __shfl_sync(all, ctl, e);
+                    const float* slot = sm.rows + e * SLOT;
+                    const Terms t = slot_terms(slot, sm.ones, el);
+                    if (PS && !(JT && (c & CTL_JOINT))) {
+                        add_terms(t, c, el, ps);
+                        if (c & CTL_LAST) {
+                            if (REC && ic.contrib) keep_pair(rec, ic, slot, ps);
+                            s += ps;
+                            ps = 0.0f;
+                        }
+                    } else {
+                        add_terms(t, c, el, s);
                     }
-            __syncthreads();
+                }
+            }
+            if (lane < SYS_STRIDE) sm.sys[bb * SYS_STRIDE + lane] = s;
+        }
+        __syncwarp();
+    }
+    __syncwarp();
+    if (lane < tile.nb) {
+        const BodyPose pose = load_pose(w, h);
+        Sys t;
+        const float* o = sm.sys + lane * SYS_STRIDE;
+#pragma unroll
+        for (int k = 0; k < 21; k++) t.h[k] = o[k];
+#pragma unroll
+        for (int k = 0; k < 6; k++) t.r[k] = o[21 + k];
+        apply_solve(w, h, pose, t);
+        if (REC && ic.contrib) record_pose(w, rec, ic.it + 1, h);
+    }
+    __syncwarp();
+}
+
+// The duals of iterations [first, end) of every pair by threads t of n, four
+// per pair; a pair without a swept body takes [unswept_first, end).
+// A pair's dual reads its two bodies at the end of an iteration, and they hold
+// still until the pair's first swept colour of the next one: there its item
+// has the constraint values at hand, so it updates the dual before it stamps
+// its rows (IterCtx::dual), and no pass over the points runs between
+// iterations.  This pass then makes up the rest after the last iteration: its
+// dual, and every iteration's for a pair that no item visits.
+template <bool REC>
+static __device__ __forceinline__ void dual_pass(const DW& w, const IterRec& rec, uint32_t t, uint32_t n, int first,
+                                                 int unswept_first, int end) {
+    const uint32_t np_all = n_pairs(w);
+    for (uint32_t i = t; i < np_all * 4u; i += n) {
+        const uint32_t p = i >> 2, np = w.p_np[p];
+        if (REC && rec.contrib && np == 0u && (i & 3u) < 2u) {  // pairs without points: zero sums
+            const uint2 ab = w.p_ab[p];
+            const uint32_t slot = (i & 3u) ? p + w.offB[ab.x + 1] : w.offA[ab.y] + w.posB[p];
+            for (int it = unswept_first; it < end && slot < rec.slots; it++)
+                for (int k = 0; k < 7; k++)
+                    rec.contrib[(size_t)it * rec.cstride + (size_t)slot * 7 + k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        if ((i & 3u) >= np) continue;
+        PairCtx c;
+        load_ctx(w, p, c);
+        const int it0 = w.colour[c.a] < 0 && w.colour[c.b] < 0 ? unswept_first : first;
+        for (uint32_t k = i & 3u; k < np; k += 4u) {
+            const uint32_t q = p * MAX_PTS + k;
+            for (int it = it0; it < end; it++) {
+                float4 lam, pen;
+                dual_point(w, c, q, lam, pen);
+                if (REC && rec.contrib) record_point(rec, it + 1, q, lam, pen);
+            }
+        }
+    }
+}
+static __device__ __forceinline__ void record_joint(const DW& w, const IterRec& rec, int it, uint32_t j) {
+    const size_t J = (size_t)w.J;
+    float4* o = rec.joint + (size_t)(it + 1) * 5 * J + j;
+    o[0] = w.j_lam_l[j];
+    o[J] = w.j_pen_l[j];
+    o[2 * J] = w.j_lam_a[j];
+    o[3 * J] = w.j_pen_a[j];
+    o[4 * J] = w.j_lim[j];
+}
+
+// Barrier over the launch's blocks, all of them resident: one block, a
+// cluster (the hardware's barrier), or a cooperative grid.  The grid's counts
+// arrivals in ctr[C_GBAR] and gives up after a bounded number of polls: the
+// error bit then reaches the host.
+// A block arrives, opens its next tiles, and then waits.
+enum SyncKind { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
+constexpr uint32_t GRID_POLLS = 1u << 23;
+static __device__ __forceinline__ void all_arrive(const DW& w, int kind) {
+    if (kind == SYNC_CLUSTER) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    } else if (kind == SYNC_GRID) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(&w.ctr[C_GBAR], 1u);
+        }
+    }
+}
+static __device__ __forceinline__ bool all_wait(const DW& w, int kind, uint32_t& target, uint32_t* ok) {
+    if (kind == SYNC_BLOCK) {
+        __syncthreads();
+        return true;
+    }
+    if (kind == SYNC_CLUSTER) {
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        return true;
+    }
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        uint32_t* bar = &w.ctr[C_GBAR];
+        uint32_t good = 1u, n = 0u;
+        while (*reinterpret_cast<volatile uint32_t*>(bar) < target)
+            if (++n > GRID_POLLS) {
+                atomicOr(&w.ctr[C_ERR], (uint32_t)E_TIMEOUT);
+                good = 0u;
+                break;
+            }
+        __threadfence();
+        *ok = good;
+    }
+    __syncthreads();
+    return *ok != 0u;
+}
+
+// REC: the instantiation of differentiable worlds, recording or not: a
+// rollout's plain and recorded passes run the same code, so they agree bit for
+// bit in the fast build too, where contraction differs from one instantiation
+// to the next.
+// Every iteration: per colour its bodies dealt over all warps of the launch,
+// a barrier, and with joints a pass over their duals.
+template <int BS, int JT, bool PS, bool REC>
+__global__ void __launch_bounds__(BS, 512 / BS) k_iterations(DW w, IterRec rec, int sync) {
+    if (aborted_solve(w)) return;
+    constexpr uint32_t NW = BS / 32;
+    extern __shared__ float4 s_dyn[];
+    WarpMem& sm = reinterpret_cast<WarpMem*>(s_dyn)[threadIdx.x >> 5];
+    __shared__ uint32_t s_ok;
+    const Elem el = elem_of(threadIdx.x & 31u);
+    const Recip rdt2 = recip_dt2(w);
+    if ((threadIdx.x & 31u) < 4u) sm.ones[threadIdx.x & 31u] = 1.0f;
+    __syncwarp();
+    const uint32_t warps = gridDim.x * NW, threads = gridDim.x * BS, tid = blockIdx.x * BS + threadIdx.x;
+    // neighbouring blocks take neighbouring tiles: warp k of block b is number k * gridDim + b
+    const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const int ncol = (int)min(w.ctr[C_NCOL], (uint32_t)MAX_COLOURS), iters = w.iterations;
+    // rolling rows read what the dual writes: with any, the dual keeps its own pass
+    const bool lazy = w.ctr[C_ROLL] == 0u;
+    if (REC && rec.contrib)
+        for (uint32_t h = tid; h < (uint32_t)w.N; h += threads)
+            if (w.colour[h] < 0)
+                for (int it = 0; it < iters; it++) record_pose(w, rec, it + 1, h);
+    __shared__ uint32_t s_col[MAX_COLOURS + 1];
+    for (uint32_t c = threadIdx.x; c <= MAX_COLOURS; c += BS) s_col[c] = w.col_cnt[c];
+    __syncthreads();
+    // bodies of colour c a warp takes at a time: every warp the same number of
+    // equal tiles, as few of up to 32 bodies as hold the colour
+    auto tile_size = [&](int c) {
+        const uint32_t n = s_col[c + 1] - s_col[c], rounds = max(1u, (n + 32u * warps - 1u) / (32u * warps));
+        return (n + rounds * warps - 1u) / (rounds * warps);
+    };
+    auto open = [&](int c, uint32_t i, uint32_t tb) {
+        const uint32_t n = s_col[c + 1] - s_col[c];
+        return open_tile<JT>(w, sm, rdt2, w.col_list, s_col[c] + i, i < n ? min(tb, n - i) : 0u);
+    };
+    if (iters <= 0) return;
+    uint32_t target = 0;
+    uint32_t tb = ncol ? tile_size(0) : 0u;
+    Tile tile = open(0, wid * tb, tb);
+    for (int it = 0; it < iters; it++) {
+        const IterCtx ic{it, lazy && it > 0,
+                         REC && rec.contrib ? reinterpret_cast<float*>(rec.contrib + (size_t)it * rec.cstride) : nullptr};
+        const bool last = it + 1 == iters;
+        for (int c = 0; c < ncol; c++) {
+            const uint32_t n = s_col[c + 1] - s_col[c];
+            for (uint32_t i = wid * tb; i < n;) {
+                solve_tile<JT, PS, REC>(w, rec, ic, sm, el, tile);
+                i += warps * tb;
+                if (i < n) tile = open(c, i, tb);
+            }
+            const int next = c + 1 < ncol ? c + 1 : 0;
+            all_arrive(w, sync);
+            if (c + 1 < ncol || !last) {
+                tb = tile_size(next);
+                tile = open(next, wid * tb, tb);
+            }
+            if (!all_wait(w, sync, target, &s_ok)) return;
+        }
+        if (!lazy || last) dual_pass<REC>(w, rec, tid, threads, it, lazy ? 0 : it, it + 1);
+        if (JT)
+            for (uint32_t j = tid; j < (uint32_t)w.J; j += threads) {
+                dual_joint<JT == 2>(w, j);
+                if (REC && ic.contrib) record_joint(w, rec, it, j);
+            }
+        if (!last && (JT || !lazy)) {
+            all_arrive(w, sync);
+            if (!all_wait(w, sync, target, &s_ok)) return;
         }
     }
 }
 
-template <int BS, int MINB, int JT>
-static void scene_solve_launch(const DW& w, cudaStream_t st) {
-    const size_t smem = (size_t)BS * 7 * sizeof(float4);
-    static int grid[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // per device ordinal
+// Blocks of kernel k that the device holds at once (per device ordinal).
+struct Resident {
+    int blocks[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+};
+template <class K>
+static int resident_blocks(Resident& r, K k, int bs, size_t smem) {
     int dev = 0;
     cudaGetDevice(&dev);
-    int& g = grid[dev & 7];
+    int& g = r.blocks[dev & 7];
     if (!g) {
-        cudaFuncSetAttribute(k_scene_solve<BS, MINB, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0, sms = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_scene_solve<BS, MINB, JT>, BS, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bs, smem);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         g = max(1, per_sm) * max(1, sms);
     }
-    k_scene_solve<BS, MINB, JT><<<min(g, max(1, w.S)), BS, smem, st>>>(w);
+    return g;
 }
-template <int JT>
-static void scene_solve_block(const DW& w, int block, cudaStream_t st) {
-    switch (block) {
-        case 128: scene_solve_launch<128, 4, JT>(w, st); break;
-        case 512: scene_solve_launch<512, 1, JT>(w, st); break;
-        default: scene_solve_launch<256, 2, JT>(w, st); break;
+template <int BS, int JT, bool PS, bool REC>
+static void iterations_launch(const DW& w, const IterRec& rec, cudaStream_t st) {
+    static Resident r;
+    const size_t smem = (BS / 32) * sizeof(WarpMem);
+    const int g = resident_blocks(r, k_iterations<BS, JT, PS, REC>, BS, smem);
+    // A block per 16 bodies (a warp per two of them: a colour is a third of a
+    // world or less).  A cluster's barrier takes 0.3 us and the grid's 1.5 us,
+    // so a small world stays within the 8 blocks of a portable cluster.
+    int blocks = max(1, min(g, (w.N + 15) / 16));
+    if (w.N <= 512) blocks = min(blocks, 8);
+    int sync = blocks == 1 ? SYNC_BLOCK : (blocks <= 8 ? SYNC_CLUSTER : SYNC_GRID);
+    if (sync != SYNC_GRID) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)blocks);
+        cfg.blockDim = dim3(BS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)blocks;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, k_iterations<BS, JT, PS, REC>, w, rec, sync);
+        return;
     }
+    cudaMemsetAsync(w.ctr + C_GBAR, 0, sizeof(uint32_t), st);
+    DW a = w;
+    IterRec b = rec;
+    void* args[] = {&a, &b, &sync};
+    cudaLaunchCooperativeKernel((const void*)k_iterations<BS, JT, PS, REC>, dim3((unsigned)blocks), dim3(BS), args, smem, st);
 }
-void launch_scene_solve(const DW& w, const Tune& tune, cudaStream_t st) {
-    cudaMemsetAsync(w.ctr + C_SCENE_Q, 0, sizeof(uint32_t), st);
-    if (!w.J) scene_solve_block<0>(w, tune.primal_block, st);
-    else if (!w.j_all) scene_solve_block<1>(w, tune.primal_block, st);
-    else scene_solve_block<2>(w, tune.primal_block, st);
+// Every iteration of the substep in the thread-per-body order (lanes 1) or
+// the split order (lanes 0, -1); r: what a rollout records of them.  A
+// differentiable world (sort_static) runs the split order, without the joint
+// kinds its reverse sweep refuses.
+void launch_iterations(const DW& w, const Tune& tune, const IterRec& r, cudaStream_t st) {
+    k_entries<<<nblk((size_t)w.N * 8, 256), 256, 0, st>>>(w);
+    const bool ps = tune.primal_lanes <= 0;
+    if (r.contrib || (w.sort_static && ps && !w.j_all)) {
+        if (!w.J) iterations_launch<256, 0, true, true>(w, r, st);
+        else iterations_launch<256, 1, true, true>(w, r, st);
+        return;
+    }
+    const int jt = !w.J ? 0 : (w.j_all ? 2 : 1);
+    if (jt == 0) ps ? iterations_launch<256, 0, true, false>(w, r, st) : iterations_launch<256, 0, false, false>(w, r, st);
+    else if (jt == 1) ps ? iterations_launch<256, 1, true, false>(w, r, st) : iterations_launch<256, 1, false, false>(w, r, st);
+    else ps ? iterations_launch<256, 2, true, false>(w, r, st) : iterations_launch<256, 2, false, false>(w, r, st);
 }
 
-// The per-scene solve's fallback for a world with a scene above its limit is
-// the split launch.
-static inline int launch_lanes(const Tune& tune) { return tune.primal_lanes < 0 ? 0 : tune.primal_lanes; }
-void launch_solve_prep(const DW& w, const Tune& tune, cudaStream_t st) {
-    if (launch_lanes(tune) != 0) return;
+void launch_side_lists(const DW& w, cudaStream_t st) {
     k_zero_u32<<<1, 256, 0, st>>>(w.side_cnt, 2 * MAX_COLOURS + 2);
     k_side_count<<<gsz(w.pair_cap, SIDE_BLOCK), SIDE_BLOCK, 0, st>>>(w);
     k_side_starts<<<1, 32, 0, st>>>(w);
     k_side_place<<<gsz(w.pair_cap, SIDE_BLOCK), SIDE_BLOCK, 0, st>>>(w);
 }
+// The lanes-per-body forms: one launch per colour.
 template <int J>
 static void primal_colour(const DW& w, const Tune& tune, int c, uint32_t max_bodies, cudaStream_t st) {
     int bs = tune.primal_block;
-    switch (launch_lanes(tune)) {
-        case 0:
-            k_side_rows<<<gsz((size_t)w.pair_cap * 2, 128), 128, 0, st>>>(w, c);
-            k_side_solve<J><<<gsz(max_bodies, 128), 128, 0, st>>>(w, c);
-            break;
-        case 1:
-            // occupancy variants of the thread-per-body kernel: 4, 6 or 8
-            // resident 128-thread blocks per SM (128, 80 or 64 registers)
-            if (tune.primal_minb >= 8) k_primal_thread<8, J><<<nblk(max_bodies, bs), bs, 0, st>>>(w, c);
-            else if (tune.primal_minb >= 6) k_primal_thread<6, J><<<nblk(max_bodies, bs), bs, 0, st>>>(w, c);
-            else k_primal_thread<4, J><<<nblk(max_bodies, bs), bs, 0, st>>>(w, c);
-            break;
+    switch (tune.primal_lanes) {
         case 4: k_primal_lanes<4, J><<<nblk((size_t)max_bodies * 4, bs), bs, 0, st>>>(w, c); break;
         case 8: k_primal_lanes<8, J><<<nblk((size_t)max_bodies * 8, bs), bs, 0, st>>>(w, c); break;
         case 16: k_primal_lanes<16, J><<<nblk((size_t)max_bodies * 16, bs), bs, 0, st>>>(w, c); break;

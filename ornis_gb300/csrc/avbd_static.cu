@@ -221,7 +221,7 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
         b.mu = cv.take<float2>(PCAP);
         b.np = cv.take<uint32_t>(PCAP);
         b.ra = cv.take<float4>((size_t)PCAP * MAX_PTS);
-        b.rb = cv.take<float4>((size_t)PCAP * MAX_PTS);
+        b.rb = cv.take<float4>((size_t)PCAP * MAX_PTS);  // follows ra without a gap: the engine's item lists span both
         b.lam = cv.take<float4>((size_t)PCAP * MAX_PTS);
         b.pen = cv.take<float4>((size_t)PCAP * MAX_PTS);
         b.roll = cv.take<float4>((size_t)PCAP * MAX_PTS);
@@ -238,6 +238,7 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
     w.boxlist = cv.take<uint32_t>(PCAP);
     w.clist = cv.take<uint32_t>(PCAP);
     w.bd_pa = cv.take<float4>(PCAP);
+    w.p_t1 = w.bd_pa;
     w.bd_pb = cv.take<float4>(PCAP);
     w.sort_key = cv.take<uint32_t>(1);
     w.sort_idx = cv.take<uint32_t>(1);
@@ -258,6 +259,7 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
     w.col_val = cv.take<uint32_t>(N);
     w.col_hist = cv.take<uint32_t>(radix_hist_words(N));
     w.ctr = cv.take<uint32_t>(C_NUM);
+    w.einfo = cv.take<uint2>(N);
     uint32_t* small = cv.take<uint32_t>(1);
     uint32_t* scan_tmp = cv.take<uint32_t>(scan_tmp_words(radix_hist_words(N) + N + 1) + 16);
     AvbdBody* stage = cv.take<AvbdBody>(N);
@@ -303,9 +305,7 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
     plan.scan_tmp = scan_tmp;
     Tune tune;  // exact build, one thread per body: the defaults of a world
     int cur = 0;
-    uint32_t ctr[C_NUM];
-    bool colour_overflow = false;  // a world reports it the same way, after finishing the substep
-    for (int s = 0; s < substeps && !colour_overflow; s++) {
+    for (int s = 0; s < substeps; s++) {
         cur = 1 - cur;  // the previous generation becomes `old`
         const Buf& c = pb[cur];
         const Buf& o = pb[1 - cur];
@@ -315,6 +315,7 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
         w.o_ab = o.ab; w.o_n = o.nn; w.o_np = o.np;
         w.oq_ra = o.ra; w.oq_rb = o.rb; w.oq_lam = o.lam; w.oq_pen = o.pen; w.oq_roll = o.roll;
         w.o_offA = o.offA;
+        w.ent = (uint2*)o.ra;
         launch_begin_substep(w, st);
         launch_wake_joint_motion(w, st);
         launch_torque(w, st);
@@ -323,23 +324,22 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
         launch_discovery(w, scan_tmp, st);
         launch_post_discovery(w, scan_tmp, st);
         launch_colouring(w, tune, scan_tmp, st);
-        if (cudaMemcpyAsync(ctr, w.ctr, sizeof(ctr), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess)
-            return AVBD_ERR_DEVICE;
-        if (ctr[C_ERR] & E_CAND_OVERFLOW) return AVBD_ERR_CAPACITY;  // more than PCAP candidates
-        if (ctr[C_ERR] & E_COLOUR_OVERFLOW) colour_overflow = true;
-        int ncol = (int)ctr[C_NCOL];
-        for (int it = 0; it < w.iterations; it++) launch_iteration(w, tune, ncol, st);
+        launch_iterations(w, tune, st);
         launch_finish_substep(w, tune, st);
     }
-    if (colour_overflow) {
-        // more colours than a launch covers: out is left untouched
-        return cudaStreamSynchronize(st) == cudaSuccess ? AVBD_ERR_CAPACITY : AVBD_ERR_DEVICE;
-    }
+    // Every kernel checks the error word on the device (an overflow stops the
+    // substep that met it and all later ones), so the host reads it once, with
+    // the records.
     k_static_out<<<1, MAXB, 0, st>>>(w, stage, N);
     if (cudaGetLastError() != cudaSuccess) return AVBD_ERR_DEVICE;
-    if (cudaMemcpyAsync(out, stage, sizeof(AvbdBody) * N, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    uint32_t ctr[C_NUM];
+    AvbdBody rec[MAXB];
+    if (cudaMemcpyAsync(ctr, w.ctr, sizeof(ctr), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaMemcpyAsync(rec, stage, sizeof(AvbdBody) * N, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return AVBD_ERR_DEVICE;
+    // more than PCAP candidates, or more colours than the solver has: out is left untouched
+    if (ctr[C_ERR] & (E_CAND_OVERFLOW | E_COLOUR_OVERFLOW)) return AVBD_ERR_CAPACITY;
+    std::memcpy(out, rec, sizeof(AvbdBody) * N);
     return AVBD_OK;
 }

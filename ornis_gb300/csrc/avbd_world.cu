@@ -285,6 +285,7 @@ static void set_pair_ptrs(AvbdWorld* W) {
     w.p_old = c.old;
     w.offA = c.offA;
     w.o_ab = o.ab; w.o_n = o.n; w.o_np = o.np;
+    w.ent = (uint2*)o.ra;
     w.oq_ra = o.ra; w.oq_rb = o.rb; w.oq_lam = o.lam; w.oq_pen = o.pen; w.oq_roll = o.roll;
     w.o_offA = o.offA;
 }
@@ -376,7 +377,8 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
         p.ab = m.get<uint2>(cand_cap); p.n = m.get<float4>(cand_cap); p.mu = m.get<float2>(cand_cap);
         p.np = m.get<uint32_t>(cand_cap);
         size_t q = (size_t)cand_cap * MAX_PTS;
-        p.ra = m.get<float4>(q); p.rb = m.get<float4>(q); p.lam = m.get<float4>(q); p.pen = m.get<float4>(q);
+        // one allocation: the tile engine keeps its item lists in the previous generation's anchors
+        p.ra = m.get<float4>(2 * q); p.rb = p.ra ? p.ra + q : nullptr; p.lam = m.get<float4>(q); p.pen = m.get<float4>(q);
         p.roll = m.get<float4>(q); p.matched = m.get<int32_t>(q);
         p.old = m.get<int32_t>(cand_cap);
         p.offA = m.get<uint32_t>(N + 1);
@@ -386,15 +388,7 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     w.posB = m.get<uint32_t>(cand_cap);
     w.side_list = m.get<uint32_t>((size_t)cand_cap * 2);
     w.side_cnt = m.get<uint32_t>(2 * MAX_COLOURS + 2);
-    // the split primal's per-incidence partial systems (the per-scene solve
-    // falls back to the split launches when a scene is above its limit)
-    uint32_t max_scene = 0;
-    for (uint32_t s = 0; s < S; s++) max_scene = std::max(max_scene, W->scene_off[s + 1] - W->scene_off[s]);
-    w.max_scene = max_scene;
-    const bool need_contrib = W->tune.primal_lanes == 0 ||
-                              (W->tune.primal_lanes < 0 && max_scene > (uint32_t)SCENE_MAX_BODIES);
-    w.contrib = need_contrib ? m.get<float4>((size_t)cand_cap * 2 * 7) : nullptr;
-    w.contrib_slots = w.contrib ? (uint32_t)(cand_cap * 2) : 0u;
+    w.einfo = m.get<uint2>(N);
     w.cand = m.get<uint2>(cand_cap);
     w.keep = m.get<uint8_t>(cand_cap);
     w.cnt = m.get<uint32_t>(N + 1);
@@ -405,6 +399,7 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     w.boxlist = m.get<uint32_t>(cand_cap);
     w.clist = m.get<uint32_t>(cand_cap);
     w.bd_pa = m.get<float4>(cand_cap);
+    w.p_t1 = w.bd_pa;
     w.bd_pb = m.get<float4>(cand_cap);
     w.aabb_lo = m.get<float4>(N); w.aabb_hi = m.get<float4>(N);
     // large-scene sort scratch
@@ -435,17 +430,6 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     W->d_small = m.get<uint32_t>(small.size());
     if (!small.empty())
         cudaMemcpy(W->d_small, small.data(), small.size() * 4, cudaMemcpyHostToDevice);
-    {
-        // the per-scene solve's queue: largest scenes first (ties by index)
-        std::vector<uint32_t> order(S);
-        for (uint32_t s = 0; s < S; s++) order[s] = s;
-        std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) {
-            return W->scene_off[a + 1] - W->scene_off[a] > W->scene_off[b + 1] - W->scene_off[b];
-        });
-        uint32_t* d = m.get<uint32_t>(S);
-        if (S) cudaMemcpy(d, order.data(), S * 4, cudaMemcpyHostToDevice);
-        w.scene_order = d;
-    }
     W->plan.small_scenes = W->d_small;
     W->plan.n_small = (int)small.size();
     w.fbody = m.get<uint32_t>(N);
@@ -1146,10 +1130,9 @@ static void enqueue_front(AvbdWorld* W, bool emit) {
 }
 static void enqueue_back(AvbdWorld* W, int ncol, bool emit) {
     const DW& w = W->w;
-    if (use_scene_solve(w, W->tune)) {
-        launch_scene_solve(w, W->tune, W->st);
+    if (use_engine(W->tune)) {
+        launch_iterations(w, W->tune, W->st);
     } else {
-        launch_solve_prep(w, W->tune, W->st);
         for (int it = 0; it < w.iterations; it++) launch_iteration(w, W->tune, ncol, W->st);
     }
     launch_finish_substep(w, W->tune, W->st);
@@ -1187,10 +1170,20 @@ static void accumulate(AvbdWorld* W) {
     W->cum.timeouts = c[C_TIMEOUT] + c[C_CCD_LEFT];
 }
 
-// One substep through plain launches (the host reads the colour count).
+// A grid barrier of the iterations gave up: the substep is not complete.
+static int timed_out(AvbdWorld* W) {
+    if (!(W->h_ctr[C_ERR] & E_TIMEOUT)) return AVBD_OK;
+    CK(cudaMemsetAsync(W->w.ctr + C_ERR, 0, 4, W->st));
+    return AVBD_ERR_TIMEOUT;
+}
+
+// One substep through plain launches (without the tile engine, the host reads the colour count).
 static int substep_plain(AvbdWorld* W, bool emit) {
     for (int attempt = 0; attempt < 8; attempt++) {
         enqueue_front(W, emit);
+        // the tile engine reads the colour count on the device
+        const bool engine = use_engine(W->tune);
+        if (engine) enqueue_back(W, 0, emit);
         CK(cudaGetLastError());
         int rc = read_ctr(W);
         if (rc) return rc;
@@ -1205,13 +1198,15 @@ static int substep_plain(AvbdWorld* W, bool emit) {
         }
         int ncol = (int)W->h_ctr[C_NCOL];
         W->last_ncol = ncol;
-        enqueue_back(W, ncol, emit);
-        CK(cudaGetLastError());
-        rc = read_ctr(W);
-        if (rc) return rc;
+        if (!engine) {
+            enqueue_back(W, ncol, emit);
+            CK(cudaGetLastError());
+            rc = read_ctr(W);
+            if (rc) return rc;
+        }
         accumulate(W);
         if (W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW) return AVBD_ERR_CAPACITY;
-        return AVBD_OK;
+        return timed_out(W);
     }
     return AVBD_ERR_CAPACITY;
 }
@@ -1246,7 +1241,6 @@ struct AdjTape {
     int nframes = 0;
     std::vector<AdjFrame> frames;
     std::vector<std::array<cudaGraphExec_t, 2>> rg;  // recording graphs per frame and parity
-    int rg_cols = 0;
     uint64_t rg_key = 0;  // the world allocation (mem_gen) the graphs were captured against
     AdjState A{};
     float ms_recompute = 0.0f, ms_reverse = 0.0f;  // device time of the last backward
@@ -1447,28 +1441,27 @@ int adj_copy_front(AvbdWorld* W, AdjTape* t, AdjFrame& f) {
     adj_copy_joints(W, f, 0);
     return AVBD_OK;
 }
-// The iterations and the finish of a substep for `cover` colours, with the
-// split primal's row sums and every iterate copied into the frame.
-int adj_back(AvbdWorld* W, AdjTape* t, AdjFrame& f, int cover) {
+// The iterations and the finish of a substep, every pair's row sums and every
+// iterate recorded into the frame on the way.
+int adj_back(AvbdWorld* W, AdjTape* t, AdjFrame& f) {
     cudaStream_t st = W->st;
     const DW& w = W->w;
-    const size_t N = (size_t)w.N, P = std::min<size_t>(t->pcap, W->cand_cap), Q = P * MAX_PTS;
-    launch_solve_prep(w, W->tune, st);
+    const size_t N = (size_t)w.N, P = std::min<size_t>(t->pcap, W->cand_cap);
+    launch_side_lists(w, W->tune, st);
     D2D(f.side_cnt, w.side_cnt, (2 * MAX_COLOURS + 2) * 4);
     D2D(f.side_list, w.side_list, P * 2 * 4);
-    for (int it = 0; it < w.iterations; it++) {
-        // the split primal writes this iteration's row sums straight into the frame
-        DW wi = w;
-        wi.contrib = f.it_contrib + it * f.cstride;
-        wi.contrib_slots = (uint32_t)(2 * P);
-        for (int c = 0; c < cover; c++) launch_primal_colour(wi, W->tune, c, (uint32_t)w.N, st);
-        D2D(f.it_pos + (it + 1) * N, w.pos, N * 16);
-        D2D(f.it_rot + (it + 1) * N, w.rot, N * 16);
-        launch_dual(w, W->tune, st);
-        D2D(f.it_lam + (it + 1) * f.qstride, w.q_lam, Q * 16);
-        D2D(f.it_pen + (it + 1) * f.qstride, w.q_pen, Q * 16);
-        adj_copy_joints(W, f, it + 1);
-    }
+    IterRec rec;
+    rec.contrib = f.it_contrib;
+    rec.cstride = f.cstride;
+    rec.slots = (uint32_t)(2 * P);
+    rec.pos = f.it_pos;
+    rec.rot = f.it_rot;
+    rec.lam = f.it_lam;
+    rec.pen = f.it_pen;
+    rec.qstride = f.qstride;
+    rec.qcap = (uint32_t)(P * MAX_PTS);
+    rec.joint = f.it_joint;
+    launch_iterations(w, W->tune, st, rec);
     launch_finish_substep(w, W->tune, st);
     D2D(f.asleep_end, w.asleep, N * 4);
     return AVBD_OK;
@@ -1486,23 +1479,18 @@ void adj_free_graphs(AdjTape* t) {
     t->rg.clear();
 }
 
-// One captured recording substep per frame and pair-buffer parity.  The
-// primal is captured for rg_cols colours; a substep that needs more is
-// finished with plain launches.
+// One captured recording substep per frame and pair-buffer parity.
 int adj_capture(AvbdWorld* W, AdjTape* t) {
     adj_free_graphs(t);
     const int base = W->cur;
-    t->rg_cols = std::max(W->graph_cols, std::max(W->last_ncol + 2, 4));
     t->rg.assign(t->frames.size(), {nullptr, nullptr});
     for (size_t k = 0; k < t->frames.size(); k++)
         for (int par = 0; par < 2; par++) {
             cudaGraph_t g;
             CK(cudaStreamBeginCapture(W->st, cudaStreamCaptureModeThreadLocal));
-            W->w.max_cols = t->rg_cols;
             enqueue_front(W, false);
             adj_copy_front(W, t, t->frames[k]);
-            adj_back(W, t, t->frames[k], t->rg_cols);
-            W->w.max_cols = MAX_COLOURS;
+            adj_back(W, t, t->frames[k]);
             CK(cudaStreamEndCapture(W->st, &g));
             cudaError_t e = cudaGraphInstantiate(&t->rg[k][W->cur], g, 0);
             cudaGraphDestroy(g);
@@ -1534,19 +1522,12 @@ int adj_substep(AvbdWorld* W, AdjTape* t, int k) {
         if (!(W->h_ctr[C_ERR] & E_CAND_OVERFLOW)) {
             const uint32_t P = W->h_ctr[C_PAIRS], ncol = W->h_ctr[C_NCOL];
             if (P > t->pcap) return AVBD_ERR_CAPACITY;
-            if (W->h_ctr[C_ERR] & E_COLOUR_RANGE) {
-                // the graph's iterations were skipped: finish this substep plainly
-                CK(cudaMemsetAsync(W->w.ctr + C_ERR, 0, 4, st));
-                adj_back(W, t, f, (int)ncol);
-                rc = read_ctr(W);
-                if (rc) return rc;
-            }
             W->last_ncol = (int)ncol;
             f.npairs = P;
             f.ncol = ncol;
             accumulate(W);
             if (W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW) return AVBD_ERR_CAPACITY;
-            return AVBD_OK;
+            return timed_out(W);
         }
         // candidate overflow: nothing after the broadphase ran; undo the flip
         // and record this substep plainly after growing
@@ -1575,13 +1556,13 @@ int adj_substep(AvbdWorld* W, AdjTape* t, int k) {
     f.npairs = P;
     f.ncol = ncol;
     adj_copy_front(W, t, f);
-    adj_back(W, t, f, (int)ncol);
+    adj_back(W, t, f);
     CK(cudaGetLastError());
     int rc = read_ctr(W);
     if (rc) return rc;
     accumulate(W);
     if (W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW) return AVBD_ERR_CAPACITY;
-    return AVBD_OK;
+    return timed_out(W);
 }
 
 int adj_reverse(AvbdWorld* W, AdjTape* t, const AdjFrame& f) {
@@ -2460,8 +2441,8 @@ static int capture(AvbdWorld* W) {
         for (int k = 0; k < 2; k++) {
             cudaGraph_t g;
             CK(cudaStreamBeginCapture(W->st, cudaStreamCaptureModeThreadLocal));
-            // the per-scene solve walks as many colours as each scene has
-            W->w.max_cols = use_scene_solve(W->w, W->tune) ? MAX_COLOURS : W->graph_cols;
+            // the tile engine walks as many colours as there are
+            W->w.max_cols = use_engine(W->tune) ? MAX_COLOURS : W->graph_cols;
             enqueue_front(W, emit != 0);
             enqueue_back(W, W->graph_cols, emit != 0);
             W->w.max_cols = MAX_COLOURS;
@@ -2488,9 +2469,10 @@ static int step_graph_n(AvbdWorld* W, int32_t substeps, bool last_only) {
     int rc = AVBD_OK;
     for (int i = 0; i < substeps; i++) {
         const bool emit = emit_at(W, i, substeps, last_only);
-        if (!W->gexec[0][0] || W->last_ncol > W->graph_cols) {
-            if (W->last_ncol == 0) {
-                rc = substep_plain(W, emit);  // learn the colour count first
+        const bool engine = use_engine(W->tune);
+        if (!W->gexec[0][0] || (!engine && W->last_ncol > W->graph_cols)) {
+            if (engine ? W->cum.steps == 0 : W->last_ncol == 0) {
+                rc = substep_plain(W, emit);  // learn the colour count first (a single step needs no graph)
                 if (rc) return rc;
                 continue;
             }
@@ -2525,6 +2507,8 @@ static int step_graph_n(AvbdWorld* W, int32_t substeps, bool last_only) {
             if (rc) return rc;
         }
         accumulate(W);
+        rc = timed_out(W);
+        if (rc) return rc;
     }
     return AVBD_OK;
 }
@@ -2677,16 +2661,6 @@ int avbd_set_tuning(AvbdWorld* W, int primal_lanes, int primal_block) {
     if (primal_lanes == 1 && primal_block > 128) return AVBD_ERR_INVALID_ARG;
     if (primal_lanes == AVBD_PRIMAL_SCENES && primal_block != 128 && primal_block != 256 && primal_block != 512)
         return AVBD_ERR_INVALID_ARG;
-    const bool need_contrib = primal_lanes == 0 ||
-                              (primal_lanes < 0 && W->w.max_scene > (uint32_t)SCENE_MAX_BODIES);
-    if (need_contrib && W->w.ctr && !W->w.contrib) {
-        // the split primal's per-incidence partial systems
-        cudaSetDevice(W->device);
-        W->w.contrib = W->mem.get<float4>((size_t)W->cand_cap * 2 * 7);
-        if (!W->w.contrib) return AVBD_ERR_DEVICE;
-        W->w.contrib_slots = (uint32_t)(W->cand_cap * 2);
-        W->mem_gen++;
-    }
     W->tune.primal_lanes = primal_lanes;
     W->tune.primal_block = primal_block;
     free_graphs(W);
@@ -2793,8 +2767,7 @@ int avbd_world_profile_substep(AvbdWorld* W, float* ms, uint32_t* info) {
     launch_post_discovery(w, W->scan_tmp, st);
     CK(cudaEventRecord(ev[5], st));
     launch_colouring(w, W->tune, W->scan_tmp, st);
-    const bool scene_solve = use_scene_solve(w, W->tune);
-    if (!scene_solve) launch_solve_prep(w, W->tune, st);
+    const bool engine = use_engine(W->tune);
     CK(cudaEventRecord(ev[6], st));
     rc = read_ctr(W);
     if (rc) return rc;
@@ -2804,15 +2777,15 @@ int avbd_world_profile_substep(AvbdWorld* W, float* ms, uint32_t* info) {
     uint32_t col_total = 0;
     CK(cudaMemcpy(&col_total, w.col_cnt + MAX_COLOURS, 4, cudaMemcpyDeviceToHost));
     float prim = 0.0f, dual = 0.0f;
-    if (scene_solve) {
+    if (engine) {
         // primal and dual of every iteration in one launch: reported as primal
         CK(cudaEventRecord(ev[6], st));
-        launch_scene_solve(w, W->tune, st);
+        launch_iterations(w, W->tune, st);
         CK(cudaEventRecord(ev[7], st));
         CK(cudaEventSynchronize(ev[7]));
         CK(cudaEventElapsedTime(&prim, ev[6], ev[7]));
     }
-    for (int it = 0; it < (scene_solve ? 0 : w.iterations); it++) {
+    for (int it = 0; it < (engine ? 0 : w.iterations); it++) {
         float t;
         CK(cudaEventRecord(ev[6], st));
         for (int c = 0; c < ncol; c++) launch_primal_colour(w, W->tune, c, (uint32_t)w.N, st);
@@ -2837,7 +2810,7 @@ int avbd_world_profile_substep(AvbdWorld* W, float* ms, uint32_t* info) {
     if (rc) return rc;
     accumulate(W);
     info[0] = (uint32_t)ncol;
-    info[1] = scene_solve ? 1u : (uint32_t)(ncol * w.iterations);
+    info[1] = engine ? 1u : (uint32_t)(ncol * w.iterations);
     info[2] = col_total;
     info[3] = W->h_ctr[C_PAIRS];
     info[4] = W->h_ctr[C_POINTS];

@@ -53,7 +53,6 @@ constexpr int MAX_PTS = AVBD_MAX_POINTS;
 constexpr int MAX_COLOURS = 64;
 constexpr int CCD_ROUNDS = 8;
 constexpr int COLOUR_ROUNDS = 24;  // device-wide colouring rounds for scenes above the one-CTA limit
-constexpr int SCENE_MAX_BODIES = 2048;  // scenes up to this size are solved by one block each (k_scene_solve)
 
 // body info word: shape kind in bits 0-3, body type in bits 4-5, trigger bit 6
 __host__ __device__ __forceinline__ uint32_t info_shape(uint32_t i) { return i & 15u; }
@@ -79,9 +78,10 @@ enum Ctr {
     C_BOXONE = 14,       // pairs with exactly one box (listed from the back of boxlist)
     C_NOBOX = 15,        // pairs without a box (clist)
     C_LONGSEG = 16,      // long static pair segments put in order by the chunk sort
-    C_SCENE_Q = 17,      // next entry of scene_order a block of the per-scene solve takes
+    C_GBAR = 17,         // arrivals at the grid barrier of the tile engine, this substep
     C_CCD_HITS = 18,     // swept-cast hits recorded this substep (ccd_hit)
-    C_NUM = 19
+    C_ROLL = 19,         // a touching pair has rolling or torsion friction (k_entries)
+    C_NUM = 20
 };
 enum ErrBits { E_CAND_OVERFLOW = 1, E_COLOUR_OVERFLOW = 2, E_TIMEOUT = 4, E_COLOUR_RANGE = 8 };
 
@@ -167,8 +167,6 @@ struct DW {
 
     const uint32_t* scene_off;  // S+1
     const uint32_t* scene_of;   // N
-    const uint32_t* scene_order;  // S: scenes by descending body count (the per-scene solve's queue)
-    uint32_t max_scene;           // bodies of the largest scene
     const uint32_t* plane_off;  // S+1: half-space bodies of each scene
     const uint32_t* plane_list;
     const HullDesc* hulls;  // convex hulls named by AVBD_SHAPE_HULL bodies (shape_params[0])
@@ -237,17 +235,21 @@ struct DW {
     uint32_t* offB;  // N+1: B-side incidence list
     uint32_t* listB;
     uint32_t* posB;  // pair -> its index in listB
-    // split primal: per-colour (pair, side) work lists and per-incidence partial systems
+    // per-colour (pair, side) lists of a recorded substep
     uint32_t* side_list;  // 2*pair_cap entries: pair * 2 + (1 for the A side, 0 for the B side)
     uint32_t* side_cnt;   // [0, MAX_COLOURS]: list starts; [MAX_COLOURS+1, 2*MAX_COLOURS+1]: cursors
-    float4* contrib;      // 7 float4 per incidence slot (21 Hessian + 6 rhs + pad)
-    uint32_t contrib_slots;  // incidence slots contrib holds
     // ... and the previous generation (read by discovery for the warm merge)
     uint2* o_ab;
     float4* o_n;
     uint32_t* o_np;
     float4 *oq_ra, *oq_rb, *oq_lam, *oq_pen, *oq_roll;
     uint32_t* o_offA;
+    // tile engine: every swept body's (point, side) items, 16 per incidence
+    // slot, in the previous generation's anchors (oq_ra and oq_rb are one
+    // allocation, dead once discovery has merged them); per body its first
+    // slot and its item count
+    uint2* ent;
+    uint2* einfo;
 
     // broadphase / discovery scratch
     uint2* cand;       // candidate (a, b), a < b
@@ -260,6 +262,7 @@ struct DW {
     uint32_t* boxlist; // box-box pair slots from the front, one-box pair slots from the back
     uint32_t* clist;   // pair slots without a box
     float4 *bd_pa, *bd_pb;  // box-box witnesses per pair slot: (pa, dist), (pb, SAT gap)
+    float4* p_t1;           // first tangent of every pair's friction frame (takes over bd_pa as each pair is built)
     float4 *aabb_lo, *aabb_hi;
     uint32_t* sort_key;
     uint32_t* sort_idx;

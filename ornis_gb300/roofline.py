@@ -15,23 +15,12 @@ iteration, independent of how the kernels stage it:
                         once per swept body)
     pair header   32 B
 
-A launch of the per-colour primal kernels covers one colour; their roofline
-uses the sum over all colours of one iteration (the same ratio as per
-launch).  The per-scene solve is one launch per substep covering every
-iteration's primal and dual: its algorithmic bytes are iterations x (primal
-+ dual bytes per iteration).  It keeps a scene's data on chip and in L2
-across the iterations, so its DRAM traffic is below these bytes.
+The tile engine is one launch per substep covering every iteration's primal
+and dual: its algorithmic bytes are iterations x (primal + dual bytes per
+iteration).  A launch of the lanes-per-body kernels covers one colour; their
+roofline uses the sum over all colours of one iteration (the same ratio as
+per launch).
 """
-
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum, one ncu capture)
-# per algorithmic byte of the split primal (k_side_rows + k_side_solve, all
-# launches of one step): 512 scenes of the batched workload at step 200,
-# exact build, 96 non-empty colour launches of each kernel moved 4,836 MB
-# against 764 MB of model bytes.  The bench scales it to its own launches by
-# the model bytes (the same mix of bodies, points and pairs per byte).
-SPLIT_TRAFFIC_PER_MODEL_BYTE = 6.33
-TRAFFIC_SOURCE = ("ncu capture (512 scenes, step 200, exact build): 6.33 DRAM bytes per model byte, "
-                  "scaled to this launch by its model bytes")
 
 PRIMAL_BODY_B = 128
 PRIMAL_POINT_B = 48
@@ -49,22 +38,19 @@ def dual_bytes_per_iteration(swept, points, pairs):
 
 
 KERNELS = {
-    "thread": "k_primal_thread (one launch per colour)",
+    "engine": "k_iterations (one launch per substep: every iteration's primal and dual)",
     "lanes": "k_primal_lanes (one launch per colour)",
-    "split": "k_side_rows + k_side_solve (one pair of launches per colour)",
-    "scene": "k_scene_solve (one launch per substep: every iteration's primal and dual, a block per scene)",
 }
 
 
-def primal_roofline(phases_ms, info, peak, kind="thread", iterations=1):
+def primal_roofline(phases_ms, info, peak, kind="engine", iterations=1):
     """Roofline entry for the primal kernel from one profiled substep.
 
-    kind: the launch that ran ("thread", "lanes", "split" — the pair of
-    kernels per colour, its time is the pair's — or "scene", the per-scene
-    solve, one launch covering every iteration's primal and dual).
+    kind: the launch that ran ("engine", one launch covering every
+    iteration's primal and dual, or "lanes", one launch per colour).
     """
     peak_gbs, source = peak
-    if kind == "scene":
+    if kind == "engine":
         b = iterations * (primal_bytes_per_iteration(info["swept"], info["points"], info["pairs"]) +
                           dual_bytes_per_iteration(info["swept"], info["points"], info["pairs"]))
         ms = phases_ms["primal"]
@@ -92,8 +78,7 @@ def primal_roofline(phases_ms, info, peak, kind="thread", iterations=1):
         "unit": "GB/s",
         "frac": achieved / peak_gbs,
         "peak_source": f"{source} (MEASURED_PEAKS.json hbm_gbs)" if source == "measured" else "fallback 6.8 TB/s",
-        "traffic": SPLIT_TRAFFIC_PER_MODEL_BYTE * b / max(1, info["colours"]) if kind == "split" else None,
-        "traffic_source": TRAFFIC_SOURCE if kind == "split" else None,
+        "traffic": None,
         "bytes_per_launch": b / max(1, info["colours"]),
         "launch_ms": per_launch_ms,
         "model": "v1: 128 B/swept body + 48 B/point + 32 B/pair per iteration",
