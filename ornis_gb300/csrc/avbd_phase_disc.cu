@@ -61,7 +61,10 @@ static __device__ __forceinline__ void discover_post(const DW& w, uint32_t a, ui
     r.separated = r.sgn > reach;
     r.keep = true;
 }
-static __device__ __noinline__ Disc discover(const DW& w, uint32_t a, uint32_t b, bool need_witness) {
+// near_boxes (the filter): set, and nothing decided, for a new box pair whose
+// gap is within reach.
+static __device__ __noinline__ Disc discover(const DW& w, uint32_t a, uint32_t b, bool need_witness,
+                                             bool* near_boxes = nullptr) {
     Disc r;
     if (!discover_pre(w, a, b, r)) return r;
     if (r.exists && !need_witness) {
@@ -79,7 +82,8 @@ static __device__ __noinline__ Disc discover(const DW& w, uint32_t a, uint32_t b
         V3 nsat;
         float gap = separating_axis(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, nsat);
         float bound = GEN_MARGIN + len(ld3(w.vel[b]) - ld3(w.vel[a])) * w.dt * 1.00001f + 1e-6f;
-        if (gap > bound) return r;
+        if (near_boxes) *near_boxes = !(gap > bound);
+        return r;
     }
     float sat = 0.0f;
     r.d = ext_distance(w, sa, sb, &sat);
@@ -110,9 +114,31 @@ static __device__ __forceinline__ void k_disc_filter_one(const DW& w, uint32_t c
         }
         return;
     }
-    Disc d = discover(w, ab.x, ab.y, false);
+    bool box = false;
+    Disc d = discover(w, ab.x, ab.y, false, &box);
+    if (box) w.boxlist[agg_inc(&w.ctr[C_BOXNEW])] = c;  // k_disc_filter_boxes decides it
     w.keep[c] = d.keep;
     if (d.keep) agg_inc_at(w.cnt, ab.x);
+}
+// New box pairs near enough to need their witness features, a warp each.
+__global__ void __launch_bounds__(128) k_disc_filter_boxes(DW w) {
+    if (aborted(w)) return;
+    const uint32_t n = w.ctr[C_BOXNEW], warps = gridDim.x * (blockDim.x / 32);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+        const uint32_t c = w.boxlist[i];
+        const uint2 ab = w.cand[c];
+        Disc r;
+        discover_pre(w, ab.x, ab.y, r);  // passed in the filter: same state, same result
+        const Shape sa = shape_of(w, ab.x), sb = shape_of(w, ab.y);
+        float sat;
+        r.d = box_box_warp(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat);
+        r.sgn = sat;
+        discover_post(w, ab.x, ab.y, sa, sb, r);
+        if ((threadIdx.x & 31u) == 0 && r.keep) {
+            w.keep[c] = 1;
+            atomicAdd(&w.cnt[ab.x], 1u);
+        }
+    }
 }
 __global__ void __launch_bounds__(128, 4) k_disc_filter(DW w, int triggers) {
     if (aborted(w)) return;
@@ -173,10 +199,8 @@ __global__ void k_sort_slots(DW w) {
 static __device__ __forceinline__ bool box_pair(const DW& w, uint2 ab) {
     return info_shape(w.info[ab.x]) == AVBD_SHAPE_BOX && info_shape(w.info[ab.y]) == AVBD_SHAPE_BOX;
 }
-// Box-box witnesses are computed ahead, one thread per box pair, into bd_pa /
-// bd_pb; the per-pair build below then reads them.  Every box pair runs the
-// same fixed loops (15 SAT axes, 16 corner and 144 edge tests), so a warp of
-// box pairs stays converged and the kernel is ALU-bound with few loads.
+// Box-box witnesses are computed ahead, a warp per box pair, into bd_pa /
+// bd_pb; the per-pair build below then reads them.
 // Pairs are built class by class (box-box, one box, no box) so the lanes of
 // a warp run the same manifold code: corners of two boxes, of one, or none.
 static __device__ __forceinline__ void k_collect_boxes_one(const DW& w, uint32_t p) {
@@ -194,15 +218,17 @@ __global__ void k_collect_boxes(DW w) {
 }
 __global__ void k_box_witness(DW w) {
     if (aborted(w)) return;
-    const uint32_t nbox = w.ctr[C_BOXPAIRS];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nbox; i += gridDim.x * blockDim.x) {
+    const uint32_t nbox = w.ctr[C_BOXPAIRS], warps = gridDim.x * (blockDim.x / 32);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nbox; i += warps) {
         uint32_t p = w.boxlist[i];
         uint2 ab = w.cand[w.slot_c[p]];
         Shape sa = shape_of(w, ab.x), sb = shape_of(w, ab.y);
         float sat;
-        Dist d = box_box(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat);
-        w.bd_pa[p] = st3(d.pa, d.dist);
-        w.bd_pb[p] = st3(d.pb, sat);
+        Dist d = box_box_warp(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat);
+        if ((threadIdx.x & 31u) == 0) {
+            w.bd_pa[p] = st3(d.pa, d.dist);
+            w.bd_pb[p] = st3(d.pb, sat);
+        }
     }
 }
 static __device__ __forceinline__ void build_pair(const DW& w, uint32_t p, uint2 ab, const Disc& d);
@@ -447,6 +473,7 @@ void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int trig
     k_zero_u32<<<g1, 256, 0, st>>>(w.cnt, w.N + 1);
     k_zero_u32<<<g1, 256, 0, st>>>(w.cur, w.N + 1);
     k_disc_filter<<<gsz(w.cand_cap, 128), 128, 0, st>>>(w, triggers && w.evs ? 1 : 0);
+    k_disc_filter_boxes<<<gsz(w.cand_cap, 4), 128, 0, st>>>(w);
     scan_exclusive(w.cnt, w.offA, w.N + 1, scan_tmp, st);
     k_place<<<gsz(w.cand_cap, 256), 256, 0, st>>>(w);
     k_sort_slots<<<nblk(w.N, 256), 256, 0, st>>>(w);
@@ -456,7 +483,7 @@ void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int trig
     }
     k_clear_flags<<<nblk(w.N, 256), 256, 0, st>>>(w);
     k_collect_boxes<<<gsz(w.pair_cap, 256), 256, 0, st>>>(w);
-    k_box_witness<<<gsz(w.pair_cap, 128), 128, 0, st>>>(w);
+    k_box_witness<<<gsz(w.pair_cap, 4), 128, 0, st>>>(w);
     for (int cls = 0; cls < 3; cls++) k_disc_build<<<gsz(w.pair_cap, 128), 128, 0, st>>>(w, cls);
 }
 

@@ -24,6 +24,8 @@ __global__ void k_begin(DW w) {
         w.ctr[C_SLEEP] = 0;
         w.ctr[C_CCD_HITS] = 0;
         w.ctr[C_ROLL] = 0;
+        w.ctr[C_BOXNEW] = 0;
+        w.ctr[C_FBOX] = 0;
         if (w.evs) w.evs[EV_TRIG_NOW] = 0;
     }
 }
@@ -587,6 +589,8 @@ struct Cast {
     V3 normal;
     V3 point;  // the target's witness at the hit
 };
+// WARP: a box against a box, every lane of a warp calling with the same bodies.
+template <bool WARP>
 static __device__ __noinline__ Cast cast_one(const DW& w, uint32_t h, uint32_t o) {
     Cast c{false, 0.0f, V0(), V0()};
     V3 disp = ld3(w.vel[h]) * w.dt;
@@ -599,7 +603,7 @@ static __device__ __noinline__ Cast cast_one(const DW& w, uint32_t h, uint32_t o
     float t = 0.0f;
     for (int it = 0; it < 24; it++) {
         mv.pos = p0 + dir * t;
-        Dist d = ext_distance(w, mv, tg, nullptr);
+        const Dist d = WARP ? box_box_warp(mv.pos, mv.rot, mv.p, tg.pos, tg.rot, tg.p, nullptr) : ext_distance(w, mv, tg, nullptr);
         if (d.dist <= SHAPE_TOUCH) {
             if (t > 0.0f) {
                 c.hit = true;
@@ -662,6 +666,7 @@ __global__ void k_ccd_init(DW w) {
 // casting again: the winner's inputs do not change between its cast and its
 // apply (a mover applies once its earlier movers are final and it has recast
 // against any that moved; later movers wait for it).
+template <bool WARP>
 static __device__ __forceinline__ void k_ccd_cast_one(const DW& w, int first, uint32_t c, uint32_t tag) {
     uint2 ab = w.cand[c];
     bool fa = w.fast[ab.x], fb = w.fast[ab.y];
@@ -672,8 +677,8 @@ static __device__ __forceinline__ void k_ccd_cast_one(const DW& w, int first, ui
         if (!first && !(w.ccd_state[h] == 0 && w.ccd_deps[h] == 0 && w.ccd_recompute[h] == 1)) continue;
         if (!ccd_target(w, h, o)) continue;
         if (!sweep_may_touch(w, h, o)) continue;
-        Cast r = cast_one(w, h, o);
-        if (r.hit) {
+        Cast r = cast_one<WARP>(w, h, o);
+        if (r.hit && (!WARP || (threadIdx.x & 31u) == 0)) {
             // earliest time wins; equal times keep the lower handle (distance.rs:886-890)
             unsigned long long key = ((unsigned long long)__float_as_uint(r.t) << 32) | o;
             atomicMin(&w.ccd_best[h], key);
@@ -700,16 +705,22 @@ __global__ void k_ccd_collect(DW w) {
         uint2 ab = w.cand[c];
         bool fa = w.fast[ab.x], fb = w.fast[ab.y];
         if (!fa && !fb) continue;
-        w.fcand[agg_inc(&w.ctr[C_FCAND])] = c;
+        if (info_shape(w.info[ab.x]) == AVBD_SHAPE_BOX && info_shape(w.info[ab.y]) == AVBD_SHAPE_BOX)
+            w.fcand[w.cand_cap - 1u - agg_inc(&w.ctr[C_FBOX])] = c;
+        else
+            w.fcand[agg_inc(&w.ctr[C_FCAND])] = c;
         if (fa && fb && ccd_target(w, ab.x, ab.y)) atomicAdd(&w.ccd_deps[ab.y], 1u);
     }
 }
 __global__ void k_ccd_cast(DW w, int first, uint32_t tag) {
     if (aborted(w)) return;
     if (w.ctr[C_FAST] == 0u || (!first && w.ctr[C_CCD_PENDING] == 0u)) return;
-    const uint32_t n = w.ctr[C_FCAND];
+    // box pairs a warp each (a cast is up to 24 distance queries in a row), the rest a thread each
+    const uint32_t n = w.ctr[C_FCAND], nb = w.ctr[C_FBOX], warps = gridDim.x * (blockDim.x / 32);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nb; i += warps)
+        k_ccd_cast_one<true>(w, first, w.fcand[w.cand_cap - 1u - i], tag);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        k_ccd_cast_one(w, first, w.fcand[i], tag);
+        k_ccd_cast_one<false>(w, first, w.fcand[i], tag);
 }
 // The record of each mover's winning cast of round `tag` (the one whose key
 // equals the mover's best; keys are unique per mover).
@@ -738,7 +749,7 @@ static __device__ void ccd_apply(const DW& w, uint32_t h, bool recorded) {
             const float4* rec = w.ccd_hit + (size_t)k * 3;
             r = Cast{true, rec[0].x, ld3(rec[1]), ld3(rec[2])};
         } else {
-            r = cast_one(w, h, o);  // the winning cast again: same inputs, same t and normal
+            r = cast_one<false>(w, h, o);  // the winning cast again: same inputs, same t and normal
         }
         V3 disp = ld3(w.vel[h]) * w.dt;
         float L = fmaxf(len(disp), MIN_TOI_DISP_LENGTH);
@@ -799,9 +810,9 @@ static __device__ __forceinline__ void k_ccd_release_one(const DW& w, int round,
 __global__ void k_ccd_release(DW w, int round) {
     if (aborted(w)) return;
     if (w.ctr[C_CCD_PENDING] == 0u) return;
-    const uint32_t n = w.ctr[C_FCAND];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        k_ccd_release_one(w, round, w.fcand[i]);
+    const uint32_t n = w.ctr[C_FCAND], m = n + w.ctr[C_FBOX];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x)
+        k_ccd_release_one(w, round, w.fcand[i < n ? i : w.cand_cap - 1u - (i - n)]);
 }
 
 __global__ void k_ccd_reset(DW w) {

@@ -81,7 +81,9 @@ enum Ctr {
     C_GBAR = 17,         // arrivals at the grid barrier of the tile engine, this substep
     C_CCD_HITS = 18,     // swept-cast hits recorded this substep (ccd_hit)
     C_ROLL = 19,         // a touching pair has rolling or torsion friction (k_entries)
-    C_NUM = 20
+    C_BOXNEW = 20,       // new box-box candidates near enough for the witness test
+    C_FBOX = 21,         // candidates with a fast body that are box pairs (listed from the back of fcand)
+    C_NUM = 22
 };
 enum ErrBits { E_CAND_OVERFLOW = 1, E_COLOUR_OVERFLOW = 2, E_TIMEOUT = 4, E_COLOUR_RANGE = 8 };
 
@@ -269,7 +271,7 @@ struct DW {
 
     // CCD scratch
     uint32_t* fbody;  // N: the fast bodies of this substep (C_FAST of them)
-    uint32_t* fcand;  // cand_cap: candidates with a fast body (C_FCAND of them)
+    uint32_t* fcand;  // cand_cap: candidates with a fast body: C_FCAND from the front, C_FBOX box pairs from the back
     uint8_t* fast;
     unsigned long long* ccd_best;
     uint32_t* ccd_deps;
