@@ -507,13 +507,102 @@ static __device__ __forceinline__ bool joint_driven(const DW& w, uint32_t j) {
     return false;
 }
 
+// ---- launches whose blocks meet at a barrier ------------------------------------
+// Barrier over a launch's blocks, all of them resident: one block, a cluster
+// (the hardware's barrier, about 0.3 us), or a cooperative grid (about 1.5
+// us).  The grid's counts arrivals in *bar, a counter that k_prologue zeroes,
+// and gives up after a bounded number of polls: the error bit then reaches
+// the host.  A block may work between its arrival and its wait.
+enum SyncKind { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
+constexpr uint32_t GRID_POLLS = 1u << 23;
+static __device__ __forceinline__ void all_arrive(uint32_t* bar, int kind) {
+    if (kind == SYNC_CLUSTER) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    } else if (kind == SYNC_GRID) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(bar, 1u);
+        }
+    }
+}
+static __device__ __forceinline__ bool all_wait(const DW& w, uint32_t* bar, int kind, uint32_t& target, uint32_t* ok) {
+    if (kind == SYNC_BLOCK) {
+        __syncthreads();
+        return true;
+    }
+    if (kind == SYNC_CLUSTER) {
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+        return true;
+    }
+    target += gridDim.x;
+    if (threadIdx.x == 0) {
+        uint32_t good = 1u, n = 0u;
+        while (*reinterpret_cast<volatile uint32_t*>(bar) < target)
+            if (++n > GRID_POLLS) {
+                atomicOr(&w.ctr[C_ERR], (uint32_t)E_TIMEOUT);
+                good = 0u;
+                break;
+            }
+        __threadfence();
+        *ok = good;
+    }
+    __syncthreads();
+    return *ok != 0u;
+}
+static __device__ __forceinline__ bool all_sync(const DW& w, uint32_t* bar, int kind, uint32_t& target, uint32_t* ok) {
+    all_arrive(bar, kind);
+    return all_wait(w, bar, kind, target, ok);
+}
+// Blocks of a kernel that the device holds at once (per device ordinal).
+struct Resident {
+    int blocks[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+};
+template <class K>
+static int resident_blocks(Resident& r, K k, int bs, size_t smem) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& g = r.blocks[dev & 7];
+    if (!g) {
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        int per_sm = 0, sms = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bs, smem);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        g = max(1, per_sm) * max(1, sms);
+    }
+    return g;
+}
+// Launch kernel k(args..., sync kind): a block per 16 bodies (a warp of the
+// iterations per two of them: a colour is a third of a world or less), never
+// more than are resident.  A small world stays within the 8 blocks of a
+// portable cluster, whose barrier is the cheaper one.
+template <class K, class... A>
+static void launch_synced(Resident& r, K k, int bs, size_t smem, int bodies, cudaStream_t st, A... args) {
+    int blocks = max(1, min(resident_blocks(r, k, bs, smem), (bodies + 15) / 16));
+    if (bodies <= 512) blocks = min(blocks, 8);
+    const int sync = blocks == 1 ? SYNC_BLOCK : (blocks <= 8 ? SYNC_CLUSTER : SYNC_GRID);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3((unsigned)bs);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    if (sync == SYNC_GRID) {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)blocks;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, args..., sync);
+}
+
 static __global__ void k_zero_u32(uint32_t* p, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) p[i] = 0u;
 }
-static __global__ void k_comp_clear(DW w) {
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h < (uint32_t)w.N) w.comp_flag[h] = 0;
-}
-
 }  // namespace avbd

@@ -208,14 +208,13 @@ __global__ void k_ev_write(DW w, int emit) {
     }
 }
 
-// the next touch set replaces the previous one: its offsets move into toff
-__global__ void k_ev_commit(DW w) {
+// The next touch set replaces the previous one (its offsets move into toff),
+// and the queue and set words move on.
+__global__ void k_ev_commit(DW w, int emit) {
     if (aborted_solve(w)) return;
     uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b <= (uint32_t)w.N) w.toff[b] = w.ev_ct[b];
-}
-__global__ void k_ev_finish(DW w, int emit) {
-    if (aborted_solve(w) || threadIdx.x != 0) return;
+    if (emit && b <= (uint32_t)w.N) w.toff[b] = w.ev_ct[b];
+    if (b != 0) return;
     const uint32_t N = (uint32_t)w.N;
     uint32_t total = w.ev_cc[N] + (emit ? w.ev_cbe[N] + w.ev_ch[N] : 0u);
     uint32_t n = w.evs[EV_N] + total;
@@ -279,13 +278,10 @@ void launch_events(const DW& w, int emit, int triggers, uint32_t* scan_tmp, cuda
     unsigned g1 = nblk((size_t)w.N + 1, 256), gb = nblk(w.N, 256);
     if (emit) k_ev_touch<<<gsz(w.pair_cap, 256), 256, 0, st>>>(w);
     k_ev_count<<<g1, 256, 0, st>>>(w, emit);
-    scan_exclusive(w.ev_cbe, w.ev_cbe, (size_t)w.N + 1, scan_tmp, st);
-    scan_exclusive(w.ev_ch, w.ev_ch, (size_t)w.N + 1, scan_tmp, st);
-    scan_exclusive(w.ev_cc, w.ev_cc, (size_t)w.N + 1, scan_tmp, st);
-    if (emit) scan_exclusive(w.ev_ct, w.ev_ct, (size_t)w.N + 1, scan_tmp, st);
+    uint32_t* counts[4] = {w.ev_cc, w.ev_cbe, w.ev_ch, w.ev_ct};
+    scan_exclusive_many(counts, emit ? 4 : 1, (size_t)w.N + 1, scan_tmp, st);
     k_ev_write<<<gb, 256, 0, st>>>(w, emit);
-    if (emit) k_ev_commit<<<g1, 256, 0, st>>>(w);
-    k_ev_finish<<<1, 32, 0, st>>>(w, emit);
+    k_ev_commit<<<emit ? g1 : 1u, 256, 0, st>>>(w, emit);
     if (emit && triggers) k_trig_events<<<1, TRIG_SORT_THREADS, 0, st>>>(w);
 }
 

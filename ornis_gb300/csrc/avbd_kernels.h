@@ -26,6 +26,9 @@ struct Tune {
 // scan_tmp_words(n) words
 size_t scan_tmp_words(size_t n);
 void scan_exclusive(const uint32_t* in, uint32_t* out, size_t n, uint32_t* tmp, cudaStream_t st);
+// the same of `count` arrays of n values, in place; tmp needs count * scan_tmp_words(n)
+constexpr int SCAN_MANY = 4;
+void scan_exclusive_many(uint32_t* const* arrays, int count, size_t n, uint32_t* tmp, cudaStream_t st);
 
 // stable LSD radix sort of (key, value) pairs, n <= capacity of the buffers
 void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, size_t n,
@@ -50,10 +53,10 @@ struct IterRec {
 };
 
 // per substep phases
-void launch_begin_substep(const DW& w, cudaStream_t st);
-void launch_wake_joint_motion(const DW& w, cudaStream_t st);
-void launch_gear_mem(const DW& w, cudaStream_t st);
-void launch_torque(const DW& w, cudaStream_t st);
+// counters, wake, gear coordinates, torque, motor and rope impulses, boxes
+void launch_prologue(const DW& w, cudaStream_t st);
+// discovery's wake votes, wake, step-start poses and targets, contact records
+void launch_post_bodies(const DW& w, cudaStream_t st);
 struct BroadphasePlan {
     const uint32_t* small_scenes = nullptr;  // device list of scenes swept by one CTA each
     int n_small = 0;
@@ -71,7 +74,6 @@ void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int trig
 void launch_post_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st);
 void launch_colouring(const DW& w, const Tune& tune, uint32_t* scan_tmp, cudaStream_t st);
 
-void launch_wake_apply(const DW& w, cudaStream_t st);
 // Contact events of this substep (emit: the step's emitting substep) and,
 // with triggers, trigger transitions; swept hits are collected every substep.
 void launch_events(const DW& w, int emit, int triggers, uint32_t* scan_tmp, cudaStream_t st);

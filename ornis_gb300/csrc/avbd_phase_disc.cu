@@ -9,8 +9,6 @@
 
 namespace avbd {
 
-void launch_wake_apply(const DW& w, cudaStream_t st);
-
 struct Disc {
     bool keep, exists, separated;
     int32_t old;  // index of the previous-generation pair, -1 when new
@@ -385,20 +383,15 @@ static __device__ __forceinline__ void build_pair(const DW& w, uint32_t p, uint2
     }
     agg_add(&w.ctr[C_POINTS], (uint32_t)nf);
 }
-// cls 0: box-box pairs, 1: one box, 2: no box
-__global__ void __launch_bounds__(128, 4) k_disc_build(DW w, int cls) {
+// cls 0: box-box pairs, 1: one box, 2: no box, side by side in one launch
+__global__ void __launch_bounds__(128, 4) k_disc_build(DW w) {
     if (aborted(w)) return;
+    const int cls = (int)blockIdx.y;
     const uint32_t n = w.ctr[cls == 0 ? C_BOXPAIRS : (cls == 1 ? C_BOXONE : C_NOBOX)];
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint32_t p = cls == 0 ? w.boxlist[i] : (cls == 1 ? w.boxlist[w.pair_cap - 1u - i] : w.clist[i]);
         k_disc_build_one(w, p);
     }
-}
-
-__global__ void k_clear_flags(DW w) {
-    if (aborted(w)) return;
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h < (uint32_t)w.N) w.flag[h] = 0;
 }
 
 // Long static segments, in (b, candidate) order: every chunk of SORT_CHUNK
@@ -469,9 +462,6 @@ __global__ void k_sort_long_rank(DW w) {
 }
 
 void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int triggers) {
-    unsigned g1 = nblk(w.N + 1, 256);
-    k_zero_u32<<<g1, 256, 0, st>>>(w.cnt, w.N + 1);
-    k_zero_u32<<<g1, 256, 0, st>>>(w.cur, w.N + 1);
     k_disc_filter<<<gsz(w.cand_cap, 128), 128, 0, st>>>(w, triggers && w.evs ? 1 : 0);
     k_disc_filter_boxes<<<gsz(w.cand_cap, 4), 128, 0, st>>>(w);
     scan_exclusive(w.cnt, w.offA, w.N + 1, scan_tmp, st);
@@ -481,30 +471,15 @@ void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int trig
         k_sort_long_chunks<<<2 * 152, 512, 0, st>>>(w);
         k_sort_long_rank<<<4 * 152, 256, 0, st>>>(w);
     }
-    k_clear_flags<<<nblk(w.N, 256), 256, 0, st>>>(w);
     k_collect_boxes<<<gsz(w.pair_cap, 256), 256, 0, st>>>(w);
     k_box_witness<<<gsz(w.pair_cap, 4), 128, 0, st>>>(w);
-    for (int cls = 0; cls < 3; cls++) k_disc_build<<<gsz(w.pair_cap, 128), 128, 0, st>>>(w, cls);
+    k_disc_build<<<dim3(gsz(w.pair_cap, 128), 3), 128, 0, st>>>(w);
 }
 
 // ---- after discovery ----------------------------------------------------------
-// mod.rs:985-992: a sleeper kicked above the thresholds wakes before warmstart
-__global__ void k_external_wake(DW w) {
-    if (aborted(w)) return;
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= (uint32_t)w.N || !w.asleep[h]) return;
-    if (len(ld3(w.vel[h])) > SLEEP_LIN || len(ld3(w.angvel[h])) > SLEEP_ANG) wake_body(w, h);
-}
 static __device__ __forceinline__ void k_countB_one(const DW& w, uint32_t p) {
     atomicAdd(&w.cnt[w.p_ab[p].y], 1u);
 }
-__global__ void k_countB(DW w) {
-    if (aborted(w)) return;
-    const uint32_t n = n_pairs(w);
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
-        k_countB_one(w, p);
-}
-
 static __device__ __forceinline__ void k_placeB_one(const DW& w, uint32_t p) {
     uint32_t b = w.p_ab[p].y;
     w.listB[w.offB[b] + atomicAdd(&w.cur[b], 1u)] = p;
@@ -533,52 +508,6 @@ __global__ void k_sortB(DW w) {
     if (w.posB)
         for (uint32_t i = s0; i < s1; i++) w.posB[w.listB[i]] = i;
 }
-// mod.rs:993-1018 (step-start pose, inertial target) and :1043-1049 (x <- y)
-__global__ void k_targets(DW w) {
-    if (aborted(w)) return;
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= (uint32_t)w.N) return;
-    float4 p = w.pos[h], q = w.rot[h];
-    if (info_type(w.info[h]) == AVBD_BODY_KINEMATIC) {
-        w.pos0[h] = w.prev_pos[h];
-        w.rot0[h] = w.prev_rot[h];
-    } else {
-        w.pos0[h] = p;
-        w.rot0[h] = q;
-    }
-    if (!solvable(w, h)) {
-        w.inertial[h] = p;
-        w.inertial_rot[h] = q;
-        return;
-    }
-    float dt = w.dt;
-    V3 y = ld3(p) + ld3(w.vel[h]) * dt + w.gravity * (dt * dt);
-    Q qt = quat_integrate(ldq(q), ld3(w.angvel[h]) * dt);
-    w.inertial[h] = st3(y, 0.0f);
-    w.inertial_rot[h] = stq(qt);
-    if (!w.asleep[h]) {
-        w.pos[h] = st3(y, 0.0f);
-        w.rot[h] = stq(qt);
-    }
-}
-// Contact record of every body for the iterations (pose, x - x0,
-// quat_diff_vec(q, q0), shape word and first parameter in one 64-byte line),
-// taken at the start of the sweep; the primal refreshes a body's record when
-// it moves it.
-__global__ void k_motion_cache(DW w) {
-    if (aborted(w)) return;
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= (uint32_t)w.N) return;
-    V3 p = ld3(w.pos[h]);
-    Q q = ldq(w.rot[h]);
-    V3 dx = p - ld3(w.pos0[h]);
-    V3 dr = quat_diff_vec(q, ldq(w.rot0[h]));
-    float4* k = w.kin + (size_t)h * 4;
-    k[0] = st3(p, w.shp[h].x);
-    k[1] = stq(q);
-    k[2] = st3(dx, __uint_as_float(w.info[h]));
-    k[3] = st3(dr, 0.0f);
-}
 // Eq. 19 warmstart decay (mod.rs:1019-1040), then the point's step-start
 // normal violation C0 (joints_ext.rs:21-32), kept in lambda.w for the
 // iterations of this substep.
@@ -601,11 +530,14 @@ static __device__ __forceinline__ void k_decay_points_one(const DW& w, uint32_t 
                              fclamp(pn.y * GAMMA, PENALTY_MIN, PENALTY_MAX),
                              fclamp(pn.z * GAMMA, PENALTY_MIN, PENALTY_MAX), 0.0f);
 }
+// With it the B-side counts of the pairs.
 __global__ void k_decay_points(DW w) {
     if (aborted(w)) return;
     const uint32_t n = n_pairs(w) * MAX_PTS;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+        if (q % MAX_PTS == 0) k_countB_one(w, q / MAX_PTS);
         k_decay_points_one(w, q);
+    }
 }
 __global__ void k_decay_joints(DW w) {
     if (aborted(w)) return;
@@ -632,20 +564,11 @@ __global__ void k_decay_joints(DW w) {
 }
 
 void launch_post_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st) {
-    unsigned gb = nblk(w.N, 256);
-    launch_wake_apply(w, st);  // discovery wake votes (rows.rs:938-941)
-    launch_wake_joint_motion(w, st);
-    k_external_wake<<<gb, 256, 0, st>>>(w);
-    unsigned g1 = nblk(w.N + 1, 256);
-    k_zero_u32<<<g1, 256, 0, st>>>(w.cnt, w.N + 1);
-    k_zero_u32<<<g1, 256, 0, st>>>(w.cur, w.N + 1);
-    k_countB<<<gsz(w.pair_cap, 256), 256, 0, st>>>(w);
+    launch_post_bodies(w, st);
+    k_decay_points<<<gsz((size_t)w.pair_cap * MAX_PTS, 256), 256, 0, st>>>(w);
     scan_exclusive(w.cnt, w.offB, w.N + 1, scan_tmp, st);
     k_placeB<<<gsz(w.pair_cap, 256), 256, 0, st>>>(w);
-    k_sortB<<<gb, 256, 0, st>>>(w);
-    k_targets<<<gb, 256, 0, st>>>(w);
-    k_motion_cache<<<gb, 256, 0, st>>>(w);
-    k_decay_points<<<gsz((size_t)w.pair_cap * MAX_PTS, 256), 256, 0, st>>>(w);
+    k_sortB<<<nblk(w.N, 256), 256, 0, st>>>(w);
     if (w.J) k_decay_joints<<<nblk(w.J, 128), 128, 0, st>>>(w);
 }
 
@@ -799,6 +722,35 @@ __global__ void k_colour_starts(DW w, int ntiles) {
     int c = threadIdx.x;
     if (c <= MAX_COLOURS) w.col_cnt[c] = w.col_hist[(size_t)c * ntiles];
 }
+// A small world's lists in one block: counts, starts, places (any order within
+// a colour: its bodies share nothing).  Up to LISTS_SMALL bodies a block's few
+// passes beat the radix path's six launches.
+constexpr int LISTS_SMALL = 4096;
+__global__ void __launch_bounds__(1024) k_colour_lists(DW w) {
+    if (aborted(w)) return;
+    __shared__ uint32_t cnt[MAX_COLOURS + 1];
+    for (int c = threadIdx.x; c <= MAX_COLOURS; c += blockDim.x) cnt[c] = 0;
+    __syncthreads();
+    for (uint32_t h = threadIdx.x; h < (uint32_t)w.N; h += blockDim.x) {
+        const int c = w.colour[h];
+        if (c >= 0) atomicAdd(&cnt[c], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t acc = 0;
+        for (int c = 0; c <= MAX_COLOURS; c++) {
+            const uint32_t n = cnt[c];
+            cnt[c] = acc;
+            w.col_cnt[c] = acc;
+            acc += n;
+        }
+    }
+    __syncthreads();
+    for (uint32_t h = threadIdx.x; h < (uint32_t)w.N; h += blockDim.x) {
+        const int c = w.colour[h];
+        if (c >= 0) w.col_list[atomicAdd(&cnt[c], 1u)] = h;
+    }
+}
 void launch_colouring(const DW& w, const Tune& tune, uint32_t* scan_tmp, cudaStream_t st) {
     const uint32_t small_max = (uint32_t)tune.small_scene_max;
     if (w.n_large_scenes) {
@@ -806,6 +758,10 @@ void launch_colouring(const DW& w, const Tune& tune, uint32_t* scan_tmp, cudaStr
         for (int r = 0; r < COLOUR_ROUNDS; r++) k_colour_round<<<gsz(w.N, 256), 256, 0, st>>>(w, small_max);
     }
     k_colour<<<w.S, 1024, 0, st>>>(w, small_max);
+    if (w.N <= LISTS_SMALL && !tune.sort_work) {
+        k_colour_lists<<<1, 1024, 0, st>>>(w);
+        return;
+    }
     k_colour_keys<<<nblk(w.N, 256), 256, 0, st>>>(w, tune.sort_work);
     int ntiles;
     if (tune.sort_work) {

@@ -1450,50 +1450,6 @@ static __device__ __forceinline__ void record_joint(const DW& w, const IterRec& 
     o[4 * J] = w.j_lim[j];
 }
 
-// Barrier over the launch's blocks, all of them resident: one block, a
-// cluster (the hardware's barrier), or a cooperative grid.  The grid's counts
-// arrivals in ctr[C_GBAR] and gives up after a bounded number of polls: the
-// error bit then reaches the host.
-// A block arrives, opens its next tiles, and then waits.
-enum SyncKind { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
-constexpr uint32_t GRID_POLLS = 1u << 23;
-static __device__ __forceinline__ void all_arrive(const DW& w, int kind) {
-    if (kind == SYNC_CLUSTER) {
-        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    } else if (kind == SYNC_GRID) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            atomicAdd(&w.ctr[C_GBAR], 1u);
-        }
-    }
-}
-static __device__ __forceinline__ bool all_wait(const DW& w, int kind, uint32_t& target, uint32_t* ok) {
-    if (kind == SYNC_BLOCK) {
-        __syncthreads();
-        return true;
-    }
-    if (kind == SYNC_CLUSTER) {
-        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-        return true;
-    }
-    target += gridDim.x;
-    if (threadIdx.x == 0) {
-        uint32_t* bar = &w.ctr[C_GBAR];
-        uint32_t good = 1u, n = 0u;
-        while (*reinterpret_cast<volatile uint32_t*>(bar) < target)
-            if (++n > GRID_POLLS) {
-                atomicOr(&w.ctr[C_ERR], (uint32_t)E_TIMEOUT);
-                good = 0u;
-                break;
-            }
-        __threadfence();
-        *ok = good;
-    }
-    __syncthreads();
-    return *ok != 0u;
-}
-
 // REC: the instantiation of differentiable worlds, recording or not: a
 // rollout's plain and recorded passes run the same code, so they agree bit for
 // bit in the fast build too, where contraction differs from one instantiation
@@ -1535,6 +1491,7 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_iterations(DW w, IterRec rec, 
         return open_tile<JT>(w, sm, rdt2, w.col_list, s_col[c] + i, i < n ? min(tb, n - i) : 0u);
     };
     if (iters <= 0) return;
+    uint32_t* bar = &w.ctr[C_GBAR];
     uint32_t target = 0;
     uint32_t tb = ncol ? tile_size(0) : 0u;
     Tile tile = open(0, wid * tb, tb);
@@ -1550,12 +1507,12 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_iterations(DW w, IterRec rec, 
                 if (i < n) tile = open(c, i, tb);
             }
             const int next = c + 1 < ncol ? c + 1 : 0;
-            all_arrive(w, sync);
+            all_arrive(bar, sync);
             if (c + 1 < ncol || !last) {
                 tb = tile_size(next);
                 tile = open(next, wid * tb, tb);
             }
-            if (!all_wait(w, sync, target, &s_ok)) return;
+            if (!all_wait(w, bar, sync, target, &s_ok)) return;
         }
         if (!lazy || last) dual_pass<REC>(w, rec, tid, threads, it, lazy ? 0 : it, it + 1);
         if (JT)
@@ -1563,63 +1520,14 @@ __global__ void __launch_bounds__(BS, 512 / BS) k_iterations(DW w, IterRec rec, 
                 dual_joint<JT == 2>(w, j);
                 if (REC && ic.contrib) record_joint(w, rec, it, j);
             }
-        if (!last && (JT || !lazy)) {
-            all_arrive(w, sync);
-            if (!all_wait(w, sync, target, &s_ok)) return;
-        }
+        if (!last && (JT || !lazy) && !all_sync(w, bar, sync, target, &s_ok)) return;
     }
 }
 
-// Blocks of kernel k that the device holds at once (per device ordinal).
-struct Resident {
-    int blocks[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-};
-template <class K>
-static int resident_blocks(Resident& r, K k, int bs, size_t smem) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int& g = r.blocks[dev & 7];
-    if (!g) {
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        int per_sm = 0, sms = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bs, smem);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        g = max(1, per_sm) * max(1, sms);
-    }
-    return g;
-}
 template <int BS, int JT, bool PS, bool REC>
 static void iterations_launch(const DW& w, const IterRec& rec, cudaStream_t st) {
     static Resident r;
-    const size_t smem = (BS / 32) * sizeof(WarpMem);
-    const int g = resident_blocks(r, k_iterations<BS, JT, PS, REC>, BS, smem);
-    // A block per 16 bodies (a warp per two of them: a colour is a third of a
-    // world or less).  A cluster's barrier takes 0.3 us and the grid's 1.5 us,
-    // so a small world stays within the 8 blocks of a portable cluster.
-    int blocks = max(1, min(g, (w.N + 15) / 16));
-    if (w.N <= 512) blocks = min(blocks, 8);
-    int sync = blocks == 1 ? SYNC_BLOCK : (blocks <= 8 ? SYNC_CLUSTER : SYNC_GRID);
-    if (sync != SYNC_GRID) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)blocks);
-        cfg.blockDim = dim3(BS);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)blocks;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, k_iterations<BS, JT, PS, REC>, w, rec, sync);
-        return;
-    }
-    cudaMemsetAsync(w.ctr + C_GBAR, 0, sizeof(uint32_t), st);
-    DW a = w;
-    IterRec b = rec;
-    void* args[] = {&a, &b, &sync};
-    cudaLaunchCooperativeKernel((const void*)k_iterations<BS, JT, PS, REC>, dim3((unsigned)blocks), dim3(BS), args, smem, st);
+    launch_synced(r, k_iterations<BS, JT, PS, REC>, BS, (BS / 32) * sizeof(WarpMem), w.N, st, w, rec);
 }
 // Every iteration of the substep in the thread-per-body order (lanes 1) or
 // the split order (lanes 0, -1); r: what a rollout records of them.  A
@@ -1674,23 +1582,21 @@ void launch_iteration(const DW& w, const Tune& tune, int ncolours, cudaStream_t 
 }
 
 // ---- BDF1 + sleep + driver baseline (mod.rs:1060-1142) -------------------------
+// flag bits for the sleep pass: 1 joint-ready, 2 supported, 4 freeze.  Every
+// writer of a flag byte within one kernel changes the same bit the same way.
 __global__ void k_bdf1(DW w) {
     if (aborted_solve(w)) return;
     uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= (uint32_t)w.N || !solved(w, h)) return;
+    if (h >= (uint32_t)w.N) return;
+    w.flag[h] = 1;
+    w.comp_flag[h] = 0;
+    if (!solved(w, h)) return;
     V3 p = ld3(w.pos[h]);
     w.vel[h] = st3((p - ld3(w.pos0[h])) / w.dt, 0.0f);
     Q q = ldq(w.rot[h]);
     V3 spin = quat_diff_vec(q, ldq(w.rot0[h]));
     w.angvel[h] = st3(len(spin) < SPIN_REST_EPS ? V0() : spin / w.dt, 0.0f);
     w.rot[h] = stq(qnormalize(q));
-}
-// flag bits for the sleep pass: 1 joint-ready, 2 supported, 4 freeze.  Every
-// writer of a flag byte within one kernel changes the same bit the same way.
-__global__ void k_ready_init(DW w) {
-    if (aborted_solve(w)) return;
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h < (uint32_t)w.N) w.flag[h] = 1;
 }
 __global__ void k_ready_joint(DW w) {
     if (aborted_solve(w)) return;
@@ -1738,10 +1644,8 @@ __global__ void k_support(DW w) {
         k_support_one(w, p);
 }
 
-__global__ void k_sleep_timer(DW w) {
-    if (aborted_solve(w)) return;
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= (uint32_t)w.N) return;
+// Sleep timer of body h; returns whether it may freeze.
+static __device__ __forceinline__ bool sleep_timer(const DW& w, uint32_t h) {
     uint8_t f = w.flag[h];
     bool freeze = w.asleep[h] != 0;
     if (solved(w, h)) {
@@ -1755,23 +1659,10 @@ __global__ void k_sleep_timer(DW w) {
             w.sleep_timer[h] = 0.0f;
         }
     }
-    w.flag[h] = freeze ? 4 : 0;
+    return freeze;
 }
-__global__ void k_freeze_gather(DW w) {
-    if (aborted_solve(w)) return;
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= (uint32_t)w.N) return;
-    int c = w.comp[h];
-    if (c >= 0 && is_dynamic(w, h) && !(w.flag[h] & 4)) w.comp_flag[c] = 1;
-}
-__global__ void k_freeze_apply(DW w, int sleep_on) {
-    if (aborted_solve(w)) return;
-    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= (uint32_t)w.N) return;
+static __device__ __forceinline__ void freeze_apply(const DW& w, uint32_t h, bool freeze, int sleep_on) {
     if (sleep_on) {
-        bool freeze = (w.flag[h] & 4) != 0;
-        int c = w.comp[h];
-        if (c >= 0 && is_dynamic(w, h) && w.comp_flag[c]) freeze = false;
         if (freeze && !w.asleep[h] && is_dynamic(w, h)) {  // sleep_staticify (body.rs:403-408)
             w.vel[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             w.angvel[h] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -1784,25 +1675,56 @@ __global__ void k_freeze_apply(DW w, int sleep_on) {
     w.prev_pos[h] = w.pos[h];
     w.prev_rot[h] = w.rot[h];
 }
+// Without joints a body freezes by itself: timer and freeze in one launch.
+__global__ void k_sleep(DW w, int sleep_on) {
+    if (aborted_solve(w)) return;
+    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= (uint32_t)w.N) return;
+    freeze_apply(w, h, sleep_on && sleep_timer(w, h), sleep_on);
+}
+__global__ void k_sleep_timer(DW w) {
+    if (aborted_solve(w)) return;
+    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= (uint32_t)w.N) return;
+    w.flag[h] = sleep_timer(w, h) ? 4 : 0;
+    w.comp_flag[h] = 0;
+}
+__global__ void k_freeze_gather(DW w) {
+    if (aborted_solve(w)) return;
+    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= (uint32_t)w.N) return;
+    int c = w.comp[h];
+    if (c >= 0 && is_dynamic(w, h) && !(w.flag[h] & 4)) w.comp_flag[c] = 1;
+}
+__global__ void k_freeze_apply(DW w) {
+    if (aborted_solve(w)) return;
+    uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h >= (uint32_t)w.N) return;
+    bool freeze = (w.flag[h] & 4) != 0;
+    int c = w.comp[h];
+    if (c >= 0 && is_dynamic(w, h) && w.comp_flag[c]) freeze = false;
+    freeze_apply(w, h, freeze, 1);
+}
 
 void launch_finish_substep(const DW& w, cudaStream_t st) {
     unsigned gb = nblk(w.N, 256);
     k_bdf1<<<gb, 256, 0, st>>>(w);
     if (w.enable_sleep) {
-        k_ready_init<<<gb, 256, 0, st>>>(w);
         if (w.J) {
             k_ready_joint<<<nblk(w.J, 128), 128, 0, st>>>(w);
-            k_comp_clear<<<gb, 256, 0, st>>>(w);
             k_ready_gather<<<gb, 256, 0, st>>>(w);
             k_ready_scatter<<<gb, 256, 0, st>>>(w);
             k_support_joints<<<nblk(w.J, 128), 128, 0, st>>>(w);
         }
         k_support<<<gsz(w.pair_cap, 256), 256, 0, st>>>(w);
-        k_sleep_timer<<<gb, 256, 0, st>>>(w);
-        k_comp_clear<<<gb, 256, 0, st>>>(w);
-        if (w.J) k_freeze_gather<<<gb, 256, 0, st>>>(w);
+        if (w.J) {
+            k_sleep_timer<<<gb, 256, 0, st>>>(w);
+            k_freeze_gather<<<gb, 256, 0, st>>>(w);
+            k_freeze_apply<<<gb, 256, 0, st>>>(w);
+            return;
+        }
     }
-    k_freeze_apply<<<gb, 256, 0, st>>>(w, w.enable_sleep);
+    k_sleep<<<gb, 256, 0, st>>>(w, w.enable_sleep);
 }
 
 }  // namespace AVBD_SOLVE_NS

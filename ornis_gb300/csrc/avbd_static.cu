@@ -316,9 +316,7 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
         w.oq_ra = o.ra; w.oq_rb = o.rb; w.oq_lam = o.lam; w.oq_pen = o.pen; w.oq_roll = o.roll;
         w.o_offA = o.offA;
         w.ent = (uint2*)o.ra;
-        launch_begin_substep(w, st);
-        launch_wake_joint_motion(w, st);
-        launch_torque(w, st);
+        launch_prologue(w, st);
         launch_broadphase(w, plan, st);
         launch_ccd(w, st);
         launch_discovery(w, scan_tmp, st);

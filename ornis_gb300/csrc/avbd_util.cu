@@ -37,18 +37,25 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* total)
     return r;
 }
 
-__global__ void k_scan_blocks(const uint32_t* in, uint32_t* out, size_t n, uint32_t* block_sums) {
+// Up to SCAN_MANY arrays of one length, an array per blockIdx.y; sums: the
+// block sums, `stride` words an array.
+struct ScanArrays {
+    const uint32_t* in[SCAN_MANY];
+    uint32_t* out[SCAN_MANY];
+};
+__global__ void k_scan_blocks(ScanArrays a, size_t n, uint32_t* sums, size_t stride) {
     __shared__ uint32_t tot;
     size_t i = (size_t)blockIdx.x * SCAN_BLOCK + threadIdx.x;
-    uint32_t v = i < n ? in[i] : 0u;
+    uint32_t v = i < n ? a.in[blockIdx.y][i] : 0u;
     uint32_t e = block_excl_scan(v, &tot);
-    if (i < n) out[i] = e;
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = tot;
+    if (i < n) a.out[blockIdx.y][i] = e;
+    if (threadIdx.x == 0) sums[blockIdx.y * stride + blockIdx.x] = tot;
 }
 
-// single block: exclusive scan of the block sums (any count, looped)
-__global__ void k_scan_sums(uint32_t* sums, size_t nb) {
+// one block per array: exclusive scan of the block sums (any count, looped)
+__global__ void k_scan_sums(uint32_t* all, size_t nb, size_t stride) {
     __shared__ uint32_t tot;
+    uint32_t* sums = all + blockIdx.x * stride;
     uint32_t carry = 0;
     for (size_t base = 0; base < nb; base += SCAN_BLOCK) {
         size_t i = base + threadIdx.x;
@@ -60,21 +67,33 @@ __global__ void k_scan_sums(uint32_t* sums, size_t nb) {
     }
 }
 
-__global__ void k_scan_add(uint32_t* out, size_t n, const uint32_t* block_sums) {
+__global__ void k_scan_add(ScanArrays a, size_t n, const uint32_t* sums, size_t stride) {
     size_t i = (size_t)blockIdx.x * SCAN_BLOCK + threadIdx.x;
-    if (i < n) out[i] += block_sums[blockIdx.x];
+    if (i < n) a.out[blockIdx.y][i] += sums[blockIdx.y * stride + blockIdx.x];
 }
 
 size_t scan_tmp_words(size_t n) { return (n + SCAN_BLOCK - 1) / SCAN_BLOCK + 1; }
 
-void scan_exclusive(const uint32_t* in, uint32_t* out, size_t n, uint32_t* tmp, cudaStream_t st) {
-    if (n == 0) return;
-    size_t nb = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
-    k_scan_blocks<<<(unsigned)nb, SCAN_BLOCK, 0, st>>>(in, out, n, tmp);
+static void scan_arrays(const ScanArrays& a, int count, size_t n, uint32_t* tmp, cudaStream_t st) {
+    if (n == 0 || count == 0) return;
+    const size_t nb = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
+    const dim3 g((unsigned)nb, (unsigned)count);
+    k_scan_blocks<<<g, SCAN_BLOCK, 0, st>>>(a, n, tmp, nb);
     if (nb > 1) {
-        k_scan_sums<<<1, SCAN_BLOCK, 0, st>>>(tmp, nb);
-        k_scan_add<<<(unsigned)nb, SCAN_BLOCK, 0, st>>>(out, n, tmp);
+        k_scan_sums<<<count, SCAN_BLOCK, 0, st>>>(tmp, nb, nb);
+        k_scan_add<<<g, SCAN_BLOCK, 0, st>>>(a, n, tmp, nb);
     }
+}
+void scan_exclusive(const uint32_t* in, uint32_t* out, size_t n, uint32_t* tmp, cudaStream_t st) {
+    ScanArrays a{};
+    a.in[0] = in;
+    a.out[0] = out;
+    scan_arrays(a, 1, n, tmp, st);
+}
+void scan_exclusive_many(uint32_t* const* arrays, int count, size_t n, uint32_t* tmp, cudaStream_t st) {
+    ScanArrays a{};
+    for (int k = 0; k < count; k++) a.in[k] = a.out[k] = arrays[k];
+    scan_arrays(a, count, n, tmp, st);
 }
 
 // ---- radix sort: 8-bit digits, tiles of RS_THREADS * RS_ITEMS keys ----------

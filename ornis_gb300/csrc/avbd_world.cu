@@ -366,7 +366,7 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     w.j_lim = m.get<float4>(J);
     w.j_ref = m.get<float4>(J); w.j_dref = m.get<float4>(J); w.j_qref = m.get<float4>(J);
     w.j_cfg = m.get<uint32_t>(J); w.j_six = m.get<float4>(3 * (size_t)J); w.j_sacc = m.get<float4>(2 * (size_t)J);
-    w.jimp_off = m.get<uint32_t>(S + 1);
+    w.jimp_off = m.get<uint32_t>(J + 1);
     w.jimp_list = m.get<uint32_t>(J);
     w.j_lam_l = m.get<float4>(J); w.j_lam_a = m.get<float4>(J); w.j_pen_l = m.get<float4>(J); w.j_pen_a = m.get<float4>(J);
     w.j_gb = m.get<uint2>(J); w.j_gmem = m.get<float4>(J); w.j_gset = m.get<uint32_t>(J);
@@ -423,7 +423,7 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     W->plan.rows = W->tune.sweep_rows;
     W->plan.row_key = m.get<uint32_t>(max_large);
     W->plan.ext = m.get<float>(W->plan.large.size());
-    size_t scan_words = std::max({scan_tmp_words((size_t)N + 1), scan_tmp_words(radix_hist_words(max_large)),
+    size_t scan_words = std::max({SCAN_MANY * scan_tmp_words((size_t)N + 1), scan_tmp_words(radix_hist_words(max_large)),
                                   scan_tmp_words(radix_hist_words(N))});
     W->scan_tmp = m.get<uint32_t>(scan_words + 16);
     W->plan.scan_tmp = W->scan_tmp;
@@ -799,21 +799,39 @@ static int upload_all(AvbdWorld* W) {
     std::vector<uint2> j_ab(J);
     std::vector<float4> j_la(J), j_lb(J), j_axa(J), j_axb(J), j_lim(J), jll(J), jla(J), jpl(J), jpa(J);
     std::vector<float4> j_ref(J), j_dref(J), j_qref(J), j_six(3 * (size_t)J), j_sacc(2 * (size_t)J);
-    // joints with a motor or a rope, per scene in joint order
-    std::vector<uint32_t> jimp_off(S + 1, 0), jimp_list;
+    // joints with a motor or a rope, grouped by the dynamic bodies they share
+    std::vector<uint32_t> jimp_off{0}, jimp_list;
     {
-        std::vector<std::vector<uint32_t>> per(S);
+        std::vector<uint32_t> root(N), imp;
+        std::iota(root.begin(), root.end(), 0u);
+        auto top = [&](uint32_t x) {
+            while (root[x] != x) x = root[x] = root[root[x]];
+            return x;
+        };
+        auto dynamic = [&](uint32_t h) { return W->bodies[h].body_type == AVBD_BODY_DYNAMIC; };
         for (uint32_t i = 0; i < J; i++) {
             const JointRec& j = W->joints[i];
-            if (j.mot_max > 0.0f || j.kind == AVBD_JOINT_ROPE || j.kind == AVBD_JOINT_MOTOR)
-                per[scene_of[j.a]].push_back(i);
+            if (!(j.mot_max > 0.0f || j.kind == AVBD_JOINT_ROPE || j.kind == AVBD_JOINT_MOTOR)) continue;
+            imp.push_back(i);
+            if (dynamic(j.a) && dynamic(j.b)) root[top(j.a)] = top(j.b);
         }
-        for (uint32_t sc = 0; sc < S; sc++) {
-            jimp_off[sc] = (uint32_t)jimp_list.size();
-            jimp_list.insert(jimp_list.end(), per[sc].begin(), per[sc].end());
+        // groups in the order of their first joint, joints in order within one
+        std::vector<int32_t> group(N, -1);
+        std::vector<std::vector<uint32_t>> per;
+        for (uint32_t i : imp) {
+            const JointRec& j = W->joints[i];
+            const uint32_t r = top(dynamic(j.a) ? j.a : j.b);
+            if (group[r] < 0) {
+                group[r] = (int32_t)per.size();
+                per.emplace_back();
+            }
+            per[group[r]].push_back(i);
         }
-        jimp_off[S] = (uint32_t)jimp_list.size();
-        w.n_imp = (int)jimp_list.size();
+        for (const auto& g : per) {
+            jimp_list.insert(jimp_list.end(), g.begin(), g.end());
+            jimp_off.push_back((uint32_t)jimp_list.size());
+        }
+        w.n_impg = (int)per.size();
     }
     for (uint32_t i = 0; i < J; i++) {
         const JointRec& j = W->joints[i];
@@ -952,7 +970,7 @@ static int upload_all(AvbdWorld* W) {
     up(w.j_ref, j_ref.data(), J * 16); up(w.j_dref, j_dref.data(), J * 16); up(w.j_qref, j_qref.data(), J * 16);
     up(w.j_cfg, j_cfg.data(), J * 4); up(w.j_six, j_six.data(), 3 * (size_t)J * 16);
     up(w.j_sacc, j_sacc.data(), 2 * (size_t)J * 16);
-    up((void*)w.jimp_off, jimp_off.data(), (S + 1) * 4);
+    up((void*)w.jimp_off, jimp_off.data(), jimp_off.size() * 4);
     up((void*)w.jimp_list, jimp_list.data(), jimp_list.size() * 4);
     up(w.j_lam_l, jll.data(), J * 16); up(w.j_lam_a, jla.data(), J * 16);
     up(w.j_pen_l, jpl.data(), J * 16); up(w.j_pen_a, jpa.data(), J * 16);
@@ -1118,10 +1136,7 @@ static void enqueue_front(AvbdWorld* W, bool emit) {
     W->cur = 1 - W->cur;  // the previous generation becomes `old`
     set_pair_ptrs(W);
     const DW& w = W->w;
-    launch_begin_substep(w, st);
-    launch_wake_joint_motion(w, st);
-    launch_gear_mem(w, st);
-    launch_torque(w, st);
+    launch_prologue(w, st);
     launch_broadphase(w, W->plan, st);
     launch_ccd(w, st);
     launch_discovery(w, W->scan_tmp, st, emit && W->has_trig);
@@ -2753,10 +2768,7 @@ int avbd_world_profile_substep(AvbdWorld* W, float* ms, uint32_t* info) {
     set_pair_ptrs(W);
     const DW& w = W->w;
     CK(cudaEventRecord(ev[0], st));
-    launch_begin_substep(w, st);
-    launch_wake_joint_motion(w, st);
-    launch_gear_mem(w, st);
-    launch_torque(w, st);
+    launch_prologue(w, st);
     CK(cudaEventRecord(ev[1], st));
     launch_broadphase(w, W->plan, st);
     CK(cudaEventRecord(ev[2], st));

@@ -83,7 +83,8 @@ enum Ctr {
     C_ROLL = 19,         // a touching pair has rolling or torsion friction (k_entries)
     C_BOXNEW = 20,       // new box-box candidates near enough for the witness test
     C_FBOX = 21,         // candidates with a fast body that are box pairs (listed from the back of fcand)
-    C_NUM = 22
+    C_CBAR = 22,         // arrivals at the grid barrier of the swept casts, this substep
+    C_NUM = 23
 };
 enum ErrBits { E_CAND_OVERFLOW = 1, E_COLOUR_OVERFLOW = 2, E_TIMEOUT = 4, E_COLOUR_RANGE = 8 };
 
@@ -220,10 +221,11 @@ struct DW {
     // per-body joint adjacency (N+1; 4J): a joint on its two bodies, a gear
     // once on each body of its coupled joints, ascending joint index
     const uint32_t *jofs, *jlist;
-    // joints with a motor or a rope, per scene in joint order (their velocity
-    // impulses run before the warm start); n_imp of them in all
+    // joints with a motor or a rope in n_impg groups connected through dynamic
+    // bodies, each in joint order (their velocity impulses run before the warm
+    // start)
     const uint32_t *jimp_off, *jimp_list;
-    int n_imp;
+    int n_impg;
 
     // contact pairs: current generation (read by the solver) ...
     uint2* p_ab;
