@@ -34,6 +34,7 @@ void scan_exclusive_many(uint32_t* const* arrays, int count, size_t n, uint32_t*
 void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t* vals_alt, size_t n,
                       uint32_t* hist, uint32_t* scan_tmp, cudaStream_t st);
 size_t radix_hist_words(size_t n);
+constexpr size_t SORT_HIST_WORDS = 304 * 256;  // digit counts of the one-launch sort's tiles
 // one stable 8-bit pass (digit = (key >> shift) & 255); hist keeps the scanned
 // digit-major table (digit d of tile t at hist[d * ntiles + t]); returns ntiles
 int radix_pass(const uint32_t* keys, const uint32_t* vals, uint32_t* okeys, uint32_t* ovals, size_t n, int shift,
@@ -60,12 +61,13 @@ void launch_post_bodies(const DW& w, cudaStream_t st);
 struct BroadphasePlan {
     const uint32_t* small_scenes = nullptr;  // device list of scenes swept by one CTA each
     int n_small = 0;
+    uint32_t small_max = 2048;  // bodies of the largest scene one CTA sorts
     std::vector<std::pair<uint32_t, uint32_t>> large;  // body ranges sorted device-wide
     uint32_t *keys_alt = nullptr, *vals_alt = nullptr, *hist = nullptr, *scan_tmp = nullptr;
     // large scenes: sweep per row of cells in Morton order (1) or one x-sweep (0)
     int rows = 1;
     uint32_t* row_key = nullptr;  // per body of the largest scene: its row's Morton code
-    float* ext = nullptr;         // per large scene: the widest AABB edge
+    float* ext = nullptr;         // per large scene: the widest AABB edge, its sort's barrier counter
 };
 void launch_broadphase(const DW& w, const BroadphasePlan& plan, cudaStream_t st);
 void launch_ccd(const DW& w, cudaStream_t st);

@@ -274,7 +274,7 @@ __global__ void k_prologue(DW w) {
     uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h == 0) {
         const int zero[] = {C_CCD_PENDING, C_BOXPAIRS, C_FCAND, C_BOXONE, C_NOBOX, C_LONGSEG, C_CAND, C_NCOL, C_FAST,
-                            C_POINTS, C_SLEEP, C_CCD_HITS, C_ROLL, C_BOXNEW, C_FBOX, C_GBAR, C_CBAR};
+                            C_POINTS, C_SLEEP, C_CCD_HITS, C_ROLL, C_BOXNEW, C_FBOX, C_GBAR, C_CBAR, C_LBAR, C_COLPEND, C_COLPEND + 1, C_COLPEND + 2, C_COLPEND + 3};
         for (int k : zero) w.ctr[k] = 0;
         if (w.evs) w.evs[EV_TRIG_NOW] = 0;
     }
@@ -393,8 +393,10 @@ static __device__ __forceinline__ bool overlap_yz(float4 alo, float4 ahi, float4
     return alo.y <= bhi.y && blo.y <= ahi.y && alo.z <= bhi.z && blo.z <= ahi.z;
 }
 
-// One CTA per small scene: bitonic sort of (min-x key, body) in shared
-// memory, then each thread sweeps forward from its sorted slot.
+// One CTA per small scene: bitonic sort of (min-x key, body) in shared memory.
+// The sorted boxes go side by side into the contact records (dead until the
+// targets are set) from the scene's first slot: (lo, body) and hi, the body ~0
+// past the last.  k_sap_small_sweep then gives every slot a warp.
 constexpr int SAP_SMALL = 2048;
 __global__ void __launch_bounds__(512) k_sap_small(DW w, const uint32_t* scenes, int nscenes) {
     __shared__ unsigned long long kv[SAP_SMALL];
@@ -431,14 +433,38 @@ __global__ void __launch_bounds__(512) k_sap_small(DW w, const uint32_t* scenes,
             }
             __syncthreads();
         }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        uint32_t a = (uint32_t)(kv[i] & 0xffffffffu);
-        float4 alo = w.aabb_lo[a], ahi = w.aabb_hi[a];
-        for (int j = i + 1; j < n; j++) {
-            uint32_t b = (uint32_t)(kv[j] & 0xffffffffu);
-            float4 blo = w.aabb_lo[b];
-            if (blo.x > ahi.x) break;
-            if (overlap_yz(alo, ahi, blo, w.aabb_hi[b])) emit_candidate(w, a, b);
+    for (uint32_t i = threadIdx.x; i < b1 - b0; i += blockDim.x) {
+        const uint32_t b = (int)i < n ? (uint32_t)(kv[i] & 0xffffffffu) : 0xffffffffu;
+        float4* o = w.kin + 2 * (size_t)(b0 + i);
+        if (b == 0xffffffffu) {
+            o[0] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(b));
+        } else {
+            o[0] = st3(ld3(w.aabb_lo[b]), __uint_as_float(b));
+            o[1] = w.aabb_hi[b];
+        }
+    }
+}
+// A warp per sorted slot tests the next 32 slots at a time until one starts
+// past its box.  Inside the sort's CTA a thread walked each slot's sweep
+// alone: 115 us for a heap of 1500 bodies, of which the sort is a tenth.
+__global__ void __launch_bounds__(256) k_sap_small_sweep(DW w, uint32_t small_max) {
+    const uint32_t lane = threadIdx.x & 31u, warps = gridDim.x * (blockDim.x / 32);
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < (uint32_t)w.N; i += warps) {
+        const uint32_t s = w.scene_of[i], end = w.scene_off[s + 1];
+        if (end - w.scene_off[s] > small_max) continue;
+        const float4 alo = w.kin[2 * (size_t)i], ahi = w.kin[2 * (size_t)i + 1];
+        const uint32_t a = __float_as_uint(alo.w);
+        if (a == 0xffffffffu) continue;
+        for (uint32_t j0 = i + 1; j0 < end; j0 += 32) {
+            const uint32_t j = j0 + lane;
+            bool past = j >= end;
+            if (!past) {
+                const float4 blo = w.kin[2 * (size_t)j];
+                const uint32_t b = __float_as_uint(blo.w);
+                past = b == 0xffffffffu || blo.x > ahi.x;
+                if (!past && overlap_yz(alo, ahi, blo, w.kin[2 * (size_t)j + 1])) emit_candidate(w, a, b);
+            }
+            if (__any_sync(0xffffffffu, past)) break;
         }
     }
 }
@@ -470,14 +496,18 @@ __global__ void k_sap_sweep(DW w, uint32_t n) {
 // Large scenes, cell rows: space is cut into cells at least as wide as the
 // scene's widest AABB (so overlapping boxes have centres in the same or
 // adjacent cells along every axis); a row is the cells of one (y, z) cell
-// pair, all x.  Bodies are sorted by (row Morton code, min x) with two
-// stable radix sorts; each body sweeps its own row forward in x as the
-// one-axis sweep does, and the four rows of the forward half of its (y, z)
-// neighbourhood over the x window its box can reach.  Every overlapping pair
-// is tested exactly once, with the same closed-interval test: the candidate
-// set is the one-axis sweep's.  Cell coordinates are taken in double from
-// the boxes' float bounds, with a 1% wider cell, so that rounding cannot
-// move a pair more than one cell apart.
+// pair, all x.  Bodies are sorted by one 32-bit key: the row's bucket (the low
+// byte of each cell coordinate, interleaved, so that neighbouring rows stay
+// near each other; rows 256 cells apart share a bucket and are told apart by
+// their full code) and the leading 16 bits of min x.  Each body sweeps its
+// own row forward in the order, and the four rows of the forward half of its
+// (y, z) neighbourhood over the x window its box can reach.  Bodies whose keys
+// agree lie in any order, so a sweep ends only past the key of its box's far
+// side and tests both x bounds: every overlapping pair is tested exactly once,
+// with the same closed-interval test, and the candidate set is the one-axis
+// sweep's.  Cell coordinates are taken in double from the boxes' float bounds,
+// with a 1% wider cell, so that rounding cannot move a pair more than one cell
+// apart.
 __device__ __forceinline__ uint32_t part1by1(uint32_t x) {
     x &= 0xffffu;
     x = (x | (x << 8)) & 0x00ff00ffu;
@@ -494,6 +524,9 @@ __device__ __forceinline__ int cell_of(double c, double cell) {
     return (int)fmin(fmax(k, 0.0), 65534.0);
 }
 __device__ __forceinline__ uint32_t row_code(int cy, int cz) { return (part1by1(cy) << 1) | part1by1(cz); }
+// the row's bucket, and the x part of a sort key
+__device__ __forceinline__ uint32_t row_bucket(int cy, int cz) { return (part1by1(cy & 255) << 1) | part1by1(cz & 255); }
+__device__ __forceinline__ uint32_t x_part(float x) { return f2key(x) >> 16; }
 __device__ __forceinline__ double row_cell(float wmax) { return 1.01 * (double)wmax; }
 __device__ __forceinline__ void row_cells(const DW& w, uint32_t h, double cell, int& cy, int& cz) {
     float4 lo = w.aabb_lo[h], hi = w.aabb_hi[h];
@@ -515,22 +548,18 @@ __global__ void k_sap_row_keys(DW w, uint32_t b0, uint32_t b1, const float* ext,
     uint32_t h = b0 + blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= b1) return;
     bool plane = unbounded_kind(info_shape(w.info[h]));
-    uint32_t rk = 0xffffffffu;
+    uint32_t rk = 0xffffffffu, key = 0xffffffffu;
     if (!plane) {
         int cy, cz;
         row_cells(w, h, row_cell(*ext), cy, cz);
         rk = row_code(cy, cz);
+        key = row_bucket(cy, cz) << 16 | x_part(w.aabb_lo[h].x);
     }
-    w.sort_key[h - b0] = plane ? 0xffffffffu : f2key(w.aabb_lo[h].x);
+    w.sort_key[h - b0] = key;
     w.sort_idx[h - b0] = h;
     row_key[h - b0] = rk;
 }
-// after the sort by min x: the row codes in that order (the second sort's keys)
-__global__ void k_sap_row_gather(DW w, uint32_t b0, uint32_t n, const uint32_t* row_key) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) w.sort_key[i] = row_key[w.sort_idx[i] - b0];
-}
-// first sorted slot in [lo, hi) whose row code is >= key
+// first sorted slot in [lo, hi) whose key is >= key
 __device__ __forceinline__ uint32_t row_lower(const uint32_t* keys, uint32_t lo, uint32_t hi, uint32_t key) {
     while (lo < hi) {
         uint32_t m = (lo + hi) >> 1;
@@ -539,46 +568,134 @@ __device__ __forceinline__ uint32_t row_lower(const uint32_t* keys, uint32_t lo,
     }
     return lo;
 }
-__global__ void k_sap_row_sweep(DW w, uint32_t n, const float* ext) {
+__global__ void k_sap_row_sweep(DW w, uint32_t b0, uint32_t n, const float* ext, const uint32_t* row_key) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t rk = w.sort_key[i];
-    if (rk == 0xffffffffu) return;  // half-spaces sort last
-    const uint32_t a = w.sort_idx[i];
+    const uint32_t a = w.sort_idx[i], rk = row_key[a - b0];
+    if (rk == 0xffffffffu) return;  // a half-space
     const float4 alo = w.aabb_lo[a], ahi = w.aabb_hi[a];
-    for (uint32_t j = i + 1; j < n && w.sort_key[j] == rk; j++) {
-        uint32_t b = w.sort_idx[j];
-        float4 blo = w.aabb_lo[b];
-        if (blo.x > ahi.x) break;
-        if (overlap_yz(alo, ahi, blo, w.aabb_hi[b])) emit_candidate(w, a, b);
-    }
+    const uint32_t xend = x_part(ahi.x);
+    // slots [j, ...) of bucket `bucket` up to the box's far side, row `row` only
+    auto sweep = [&](uint32_t j, uint32_t bucket, uint32_t row) {
+        for (; j < n; j++) {
+            const uint32_t k = w.sort_key[j];
+            if (k >> 16 != bucket || (k & 0xffffu) > xend) break;
+            const uint32_t b = w.sort_idx[j];
+            if (row_key[b - b0] != row) continue;
+            const float4 blo = w.aabb_lo[b], bhi = w.aabb_hi[b];
+            if (alo.x <= bhi.x && blo.x <= ahi.x && overlap_yz(alo, ahi, blo, bhi)) emit_candidate(w, a, b);
+        }
+    };
     const float wmax = *ext;
     int cy, cz;
     row_cells(w, a, row_cell(wmax), cy, cz);
+    sweep(i + 1, row_bucket(cy, cz), rk);
     // a neighbour's box reaches x >= alo.x only if its min x is at least this
     const double reach = (double)alo.x - 1.01 * (double)wmax - 1e-6 * fabs((double)alo.x);
+    const uint32_t xbegin = x_part(__double2float_rd(reach));
     const int dy[4] = {0, 1, 1, 1}, dz[4] = {1, -1, 0, 1};
     for (int k = 0; k < 4; k++) {
         int ny = cy + dy[k], nz = cz + dz[k];
         if (ny > 65534 || nz < 0 || nz > 65534) continue;
-        const uint32_t nk = row_code(ny, nz);
-        uint32_t r0 = row_lower(w.sort_key, 0, n, nk);
-        uint32_t r1 = row_lower(w.sort_key, r0, n, nk + 1u);
-        // first slot of the row whose min x reaches the window
-        uint32_t lo = r0, hi = r1;
-        while (lo < hi) {
-            uint32_t m = (lo + hi) >> 1;
-            if ((double)w.aabb_lo[w.sort_idx[m]].x < reach) lo = m + 1;
-            else hi = m;
-        }
-        for (uint32_t j = lo; j < r1; j++) {
-            uint32_t b = w.sort_idx[j];
-            float4 blo = w.aabb_lo[b];
-            if (blo.x > ahi.x) break;
-            float4 bhi = w.aabb_hi[b];
-            if (alo.x <= bhi.x && overlap_yz(alo, ahi, blo, bhi)) emit_candidate(w, a, b);
-        }
+        const uint32_t bucket = row_bucket(ny, nz);
+        sweep(row_lower(w.sort_key, 0, n, bucket << 16 | xbegin), bucket, row_code(ny, nz));
     }
+}
+
+// ---- the rows' sort in one launch --------------------------------------------------
+// Stable LSD radix sort of (sort_key, sort_idx), four 8-bit passes, a barrier
+// after a pass's digit counts and after its scatter.  As launches, a pass is
+// five (0.22 ms for the 45,000 bodies of a ragdoll scene, nearly all of it
+// launches and half-empty grids); here tiles are as small as gives every
+// block one, and a block adds up the counts before it itself, which is why the
+// launch form takes over above SORT_TILES tiles of 8 x 256 keys.
+constexpr int SORT_TILES = 304;
+struct SortBufs {
+    uint32_t *k0, *v0, *k1, *v1, *hist;
+};
+__global__ void __launch_bounds__(256) k_sap_sort(DW w, SortBufs sb, uint32_t n, uint32_t rounds, uint32_t* bar, int sync) {
+    __shared__ uint32_t base[256], cnt[8][256], wsum[8], s_ok;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, ntiles = gridDim.x;
+    const uint32_t first = blockIdx.x * rounds * 256u;
+    uint32_t target = 0;
+    for (int pass = 0; pass < 4; pass++) {
+        const int shift = 8 * pass;
+        const uint32_t *ki = pass & 1 ? sb.k1 : sb.k0, *vi = pass & 1 ? sb.v1 : sb.v0;
+        uint32_t *ko = pass & 1 ? sb.k0 : sb.k1, *vo = pass & 1 ? sb.v0 : sb.v1;
+        base[tid] = 0;
+        __syncthreads();
+        for (uint32_t r = 0; r < rounds; r++) {
+            const uint32_t i = first + r * 256u + tid;
+            if (i < n) atomicAdd(&base[(ki[i] >> shift) & 255u], 1u);
+        }
+        __syncthreads();
+        sb.hist[blockIdx.x * 256u + tid] = base[tid];
+        if (!all_sync(w, bar, sync, target, &s_ok)) return;
+        // thread d: keys of digit d in all tiles, and in the tiles before this one
+        uint32_t total = 0, before = 0;
+        for (uint32_t t = 0; t < ntiles; t++) {
+            const uint32_t v = sb.hist[t * 256u + tid];
+            if (t < blockIdx.x) before += v;
+            total += v;
+        }
+        uint32_t inc = total;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= (uint32_t)o) inc += v;
+        }
+        if (lane == 31) wsum[wid] = inc;
+        __syncthreads();
+        uint32_t off = inc - total + before;
+        for (uint32_t k = 0; k < wid; k++) off += wsum[k];
+        base[tid] = off;
+        for (uint32_t r = 0; r < rounds; r++) {
+            for (int k = 0; k < 8; k++) cnt[k][tid] = 0;
+            __syncthreads();
+            const uint32_t i = first + r * 256u + tid;
+            const bool valid = i < n;
+            const uint32_t key = valid ? ki[i] : 0u, d = valid ? (key >> shift) & 255u : 256u;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d), rank = __popc(peers & ((1u << lane) - 1u));
+            if (valid && rank == 0) cnt[wid][d] = __popc(peers);
+            __syncthreads();
+            if (valid) {
+                uint32_t o = base[d] + rank;
+                for (uint32_t k = 0; k < wid; k++) o += cnt[k][d];
+                ko[o] = key;
+                vo[o] = vi[i];
+            }
+            __syncthreads();
+            uint32_t add = 0;
+            for (int k = 0; k < 8; k++) add += cnt[k][tid];
+            base[tid] += add;
+            __syncthreads();
+        }
+        if (pass < 3 && !all_sync(w, bar, sync, target, &s_ok)) return;
+    }
+}
+static void launch_row_sort(const DW& w, const BroadphasePlan& plan, uint32_t n, uint32_t* bar, cudaStream_t st) {
+    const uint32_t rounds = (n + SORT_TILES * 256u - 1) / (SORT_TILES * 256u);
+    if (rounds > 8u) {
+        radix_sort_pairs(w.sort_key, w.sort_idx, plan.keys_alt, plan.vals_alt, n, plan.hist, plan.scan_tmp, st);
+        return;
+    }
+    static Resident r;
+    const uint32_t tiles = (n + rounds * 256u - 1) / (rounds * 256u);
+    if ((int)tiles > resident_blocks(r, k_sap_sort, 256, 0)) {
+        radix_sort_pairs(w.sort_key, w.sort_idx, plan.keys_alt, plan.vals_alt, n, plan.hist, plan.scan_tmp, st);
+        return;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_sap_sort, w, SortBufs{w.sort_key, w.sort_idx, plan.keys_alt, plan.vals_alt, plan.hist}, n,
+                       rounds, bar, (int)SYNC_GRID);
 }
 
 // Swept-cast state of body h, and the list of the fast bodies.
@@ -639,19 +756,21 @@ __global__ void k_plane_cands(DW w) {
 
 void launch_broadphase(const DW& w, const BroadphasePlan& plan, cudaStream_t st) {
     k_plane_cands<<<nblk((size_t)w.N + 1, 256), 256, 0, st>>>(w);
-    if (plan.n_small) k_sap_small<<<plan.n_small, 512, 0, st>>>(w, plan.small_scenes, plan.n_small);
+    if (plan.n_small) {
+        k_sap_small<<<plan.n_small, 512, 0, st>>>(w, plan.small_scenes, plan.n_small);
+        k_sap_small_sweep<<<gsz((size_t)w.N * 32, 256), 256, 0, st>>>(w, plan.small_max);
+    }
+    // per large scene its widest box edge and its sort's barrier counter
+    if (plan.rows && !plan.large.empty()) cudaMemsetAsync(plan.ext, 0, plan.large.size() * 2 * sizeof(float), st);
     for (size_t i = 0; i < plan.large.size(); i++) {
         uint32_t b0 = plan.large[i].first, b1 = plan.large[i].second;
         uint32_t n = b1 - b0;
         if (plan.rows) {
-            float* ext = plan.ext + i;
-            cudaMemsetAsync(ext, 0, sizeof(float), st);
+            float* ext = plan.ext + 2 * i;
             k_sap_extent<<<std::min<unsigned>(nblk(n, 256), 4u * 152u), 256, 0, st>>>(w, b0, b1, ext);
             k_sap_row_keys<<<nblk(n, 256), 256, 0, st>>>(w, b0, b1, ext, plan.row_key);
-            radix_sort_pairs(w.sort_key, w.sort_idx, plan.keys_alt, plan.vals_alt, n, plan.hist, plan.scan_tmp, st);
-            k_sap_row_gather<<<nblk(n, 256), 256, 0, st>>>(w, b0, n, plan.row_key);
-            radix_sort_pairs(w.sort_key, w.sort_idx, plan.keys_alt, plan.vals_alt, n, plan.hist, plan.scan_tmp, st);
-            k_sap_row_sweep<<<nblk(n, 128), 128, 0, st>>>(w, n, ext);
+            launch_row_sort(w, plan, n, (uint32_t*)(ext + 1), st);
+            k_sap_row_sweep<<<nblk(n, 128), 128, 0, st>>>(w, b0, n, ext, plan.row_key);
             continue;
         }
         k_sap_keys<<<nblk(n, 256), 256, 0, st>>>(w, b0, b1);

@@ -419,10 +419,10 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     w.sort_idx = m.get<uint32_t>(max_large);
     W->plan.keys_alt = m.get<uint32_t>(max_large);
     W->plan.vals_alt = m.get<uint32_t>(max_large);
-    W->plan.hist = m.get<uint32_t>(radix_hist_words(max_large));
+    W->plan.hist = m.get<uint32_t>(std::max<size_t>(radix_hist_words(max_large), SORT_HIST_WORDS));
     W->plan.rows = W->tune.sweep_rows;
     W->plan.row_key = m.get<uint32_t>(max_large);
-    W->plan.ext = m.get<float>(W->plan.large.size());
+    W->plan.ext = m.get<float>(2 * W->plan.large.size());
     size_t scan_words = std::max({SCAN_MANY * scan_tmp_words((size_t)N + 1), scan_tmp_words(radix_hist_words(max_large)),
                                   scan_tmp_words(radix_hist_words(N))});
     W->scan_tmp = m.get<uint32_t>(scan_words + 16);
@@ -432,6 +432,7 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
         cudaMemcpy(W->d_small, small.data(), small.size() * 4, cudaMemcpyHostToDevice);
     W->plan.small_scenes = W->d_small;
     W->plan.n_small = (int)small.size();
+    W->plan.small_max = (uint32_t)W->tune.small_scene_max;
     w.fbody = m.get<uint32_t>(N);
     w.fcand = m.get<uint32_t>(cand_cap);
     w.fast = m.get<uint8_t>(N);

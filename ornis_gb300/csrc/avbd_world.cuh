@@ -52,7 +52,6 @@ constexpr float POS_CORRECTION_EPS = 1e-6f;  // constants.rs:71
 constexpr int MAX_PTS = AVBD_MAX_POINTS;
 constexpr int MAX_COLOURS = 64;
 constexpr int CCD_ROUNDS = 8;
-constexpr int COLOUR_ROUNDS = 24;  // device-wide colouring rounds for scenes above the one-CTA limit
 
 // body info word: shape kind in bits 0-3, body type in bits 4-5, trigger bit 6
 __host__ __device__ __forceinline__ uint32_t info_shape(uint32_t i) { return i & 15u; }
@@ -84,7 +83,9 @@ enum Ctr {
     C_BOXNEW = 20,       // new box-box candidates near enough for the witness test
     C_FBOX = 21,         // candidates with a fast body that are box pairs (listed from the back of fcand)
     C_CBAR = 22,         // arrivals at the grid barrier of the swept casts, this substep
-    C_NUM = 23
+    C_LBAR = 23,         // arrivals at the grid barrier of the large scenes' colouring, this substep
+    C_COLPEND = 24,      // four words: a body is uncoloured after round r (word r mod 4)
+    C_NUM = 28
 };
 enum ErrBits { E_CAND_OVERFLOW = 1, E_COLOUR_OVERFLOW = 2, E_TIMEOUT = 4, E_COLOUR_RANGE = 8 };
 
