@@ -114,9 +114,53 @@ static __device__ __forceinline__ void local_window(const Shape& convex, V3 pos,
         hi = V3{fmaxf(hi.x, l.x), fmaxf(hi.y, l.y), fmaxf(hi.z, l.z)};
     }
 }
+// A wide query (terrain, mesh, compound) takes the nearest of several convex
+// queries: the loops keep the first, then every strictly nearer one.  Dealt
+// over a warp, query k to lane k mod 32, the winner is the nearest of the
+// lowest k, and query 0 if its distance is not a number.
+static __device__ __forceinline__ bool wide_kind(uint32_t k) {
+    return k == AVBD_SHAPE_HEIGHTFIELD || k == AVBD_SHAPE_TRIMESH || k == AVBD_SHAPE_COMPOUND;
+}
+static __device__ __forceinline__ bool wide_pair(uint32_t ka, uint32_t kb) { return wide_kind(ka) || wide_kind(kb); }
+template <bool ON>
+struct Wide {
+    static constexpr bool on = ON;
+};
+struct Nearest {
+    Dist best;
+    uint32_t at;  // 0xffffffff: none
+    __device__ void take(uint32_t k, const Dist& d) {
+        if (k == 0u || (at == 0xffffffffu ? d.dist == d.dist : d.dist < best.dist)) {
+            best = d;
+            at = k;
+        }
+    }
+    __device__ void over_warp() {
+        const uint32_t all = 0xffffffffu;
+        const uint32_t stuck = __shfl_sync(all, (uint32_t)(at == 0u && best.dist != best.dist), 0);
+        float g0 = best.dist;
+        uint32_t win = at;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float g = __shfl_xor_sync(all, g0, o);
+            const uint32_t i = __shfl_xor_sync(all, win, o);
+            if (i != 0xffffffffu && (win == 0xffffffffu || g < g0 || (g == g0 && i < win))) {
+                g0 = g;
+                win = i;
+            }
+        }
+        at = stuck ? 0u : win;
+        const int src = (int)(at & 31u);
+        auto pick = [&](float v) { return __shfl_sync(all, v, src); };
+        best = {pick(best.dist), V3{pick(best.pa.x), pick(best.pa.y), pick(best.pa.z)},
+                V3{pick(best.pb.x), pick(best.pb.y), pick(best.pb.z)}};
+    }
+};
 // heightfield_convex (distance.rs:246-350): the nearest overlapped column,
 // each a solid box from the lowest sample up to its height (a flat one a
-// one-cell skirt); `first`: the terrain owns pa.
+// one-cell skirt); `first`: the terrain owns pa.  WARP: every lane of a warp
+// calls with the same arguments and gets the same result.
+template <bool WARP>
 static __device__ __noinline__ Dist hf_convex(const DW& w, const Shape& t, const Shape& convex, bool first) {
     const HfDesc hf = w.hfs[(uint32_t)t.p.x];
     V3 lo, hi;
@@ -132,29 +176,43 @@ static __device__ __noinline__ Dist hf_convex(const DW& w, const Shape& t, const
     const float x_origin = -(float)(hf.cols - 1) * HALF * hf.cell, z_origin = -(float)(hf.rows - 1) * HALF * hf.cell;
     bool have = false;
     Dist best{INFINITY, t.pos, convex.pos};
-    for (uint32_t row = r0; row <= r1; row++)
-        for (uint32_t col = c0; col <= c1; col++) {
-            const float h = hf.h[(size_t)row * hf.cols + col];
-            const float y_low = h - hf.y_min >= 1e-4f ? hf.y_min : h - fmaxf(hf.cell, 1e-3f);
-            const V3 mn{x_origin + (float)col * hf.cell, y_low, z_origin + (float)row * hf.cell};
-            const V3 mx{mn.x + hf.cell, fmaxf(h, y_low), mn.z + hf.cell};
-            const V3 center = (mn + mx) * HALF;
-            V3 hl = (mx - mn) * HALF;
-            hl = V3{fmaxf(hl.x, 0.0f), fmaxf(hl.y, 0.0f), fmaxf(hl.z, 0.0f)};
-            const Shape column{AVBD_SHAPE_BOX, hl, t.pos + qrot(t.rot, center), t.rot, nullptr};
-            const Dist d = shape_distance(column, convex, nullptr);
-            if (!have || d.dist < best.dist) {
-                best = d;
-                have = true;
+    auto query = [&](uint32_t row, uint32_t col) {
+        const float h = hf.h[(size_t)row * hf.cols + col];
+        const float y_low = h - hf.y_min >= 1e-4f ? hf.y_min : h - fmaxf(hf.cell, 1e-3f);
+        const V3 mn{x_origin + (float)col * hf.cell, y_low, z_origin + (float)row * hf.cell};
+        const V3 mx{mn.x + hf.cell, fmaxf(h, y_low), mn.z + hf.cell};
+        const V3 center = (mn + mx) * HALF;
+        V3 hl = (mx - mn) * HALF;
+        hl = V3{fmaxf(hl.x, 0.0f), fmaxf(hl.y, 0.0f), fmaxf(hl.z, 0.0f)};
+        const Shape column{AVBD_SHAPE_BOX, hl, t.pos + qrot(t.rot, center), t.rot, nullptr};
+        return shape_distance(column, convex, nullptr);
+    };
+    if (WARP) {
+        const uint32_t nc = c1 >= c0 ? c1 - c0 + 1u : 0u, n = r1 >= r0 ? nc * (r1 - r0 + 1u) : 0u;
+        Nearest near{best, 0xffffffffu};
+        for (uint32_t k = threadIdx.x & 31u; k < n; k += 32u) near.take(k, query(r0 + k / nc, c0 + k % nc));
+        near.over_warp();
+        have = n > 0u;
+        best = near.best;
+    } else {
+        for (uint32_t row = r0; row <= r1; row++)
+            for (uint32_t col = c0; col <= c1; col++) {
+                const Dist d = query(row, col);
+                if (!have || d.dist < best.dist) {
+                    best = d;
+                    have = true;
+                }
             }
-        }
+    }
     if (!have) return first ? Dist{INFINITY, t.pos, convex.pos} : Dist{INFINITY, convex.pos, t.pos};
     return first ? best : Dist{best.dist, best.pb, best.pa};
 }
 // trimesh_convex (distance.rs:416-517): the nearest triangle whose tree
 // boxes overlap the convex side's window, walked last-in-first-out; the
 // winner's witnesses come back swapped when the mesh is the first shape and
-// as found when it is the second (the reference's own order, kept).
+// as found when it is the second (the reference's own order, kept).  WARP:
+// the lanes walk the tree together and take 32 triangles at a time.
+template <bool WARP>
 static __device__ __noinline__ Dist mesh_convex(const DW& w, const Shape& m, const Shape& convex, bool first) {
     const MeshDesc mesh = w.meshes[(uint32_t)m.p.x];
     const Dist none = first ? Dist{INFINITY, m.pos, convex.pos} : Dist{INFINITY, convex.pos, m.pos};
@@ -163,6 +221,12 @@ static __device__ __noinline__ Dist mesh_convex(const DW& w, const Shape& m, con
     local_window(convex, m.pos, m.rot, lo, hi);
     bool have = false;
     Dist best = none;
+    auto query = [&](uint32_t tri) {
+        const Shape th{AVBD_SHAPE_HULL, V0(), m.pos + qrot(m.rot, ld3(mesh.cent[tri])), m.rot, &mesh.tris[tri]};
+        return shape_distance(th, convex, nullptr);
+    };
+    Nearest near{best, 0xffffffffu};
+    uint32_t k = 0, mine = 0;  // WARP: triangles so far; this lane's of the last 32
     uint32_t stack[64];
     uint32_t len = 1;
     stack[0] = 0;
@@ -178,8 +242,12 @@ static __device__ __noinline__ Dist mesh_convex(const DW& w, const Shape& m, con
             for (uint32_t o = node.a; o < end; o++) {
                 const uint32_t tri = mesh.order[o];
                 if (tri >= mesh.ntris) continue;
-                const Shape th{AVBD_SHAPE_HULL, V0(), m.pos + qrot(m.rot, ld3(mesh.cent[tri])), m.rot, &mesh.tris[tri]};
-                const Dist d = shape_distance(th, convex, nullptr);
+                if (WARP) {
+                    if ((k & 31u) == (threadIdx.x & 31u)) mine = tri;
+                    if ((++k & 31u) == 0u) near.take(k - 32u + (threadIdx.x & 31u), query(mine));
+                    continue;
+                }
+                const Dist d = query(tri);
                 if (!have || d.dist < best.dist) {
                     best = d;
                     have = true;
@@ -192,21 +260,28 @@ static __device__ __noinline__ Dist mesh_convex(const DW& w, const Shape& m, con
             len += 2;
         }
     }
+    if (WARP) {
+        if ((threadIdx.x & 31u) < (k & 31u)) near.take((k & ~31u) + (threadIdx.x & 31u), query(mine));
+        near.over_warp();
+        have = k > 0u;
+        best = near.best;
+    }
     if (!have) return none;
     return first ? Dist{best.dist, best.pb, best.pa} : best;
 }
 // shape_distance below the rounded and compound arms (distance.rs:706-745):
 // half-spaces, terrain, meshes, then the primitive pairs.
+template <bool WARP>
 static __device__ __noinline__ Dist leaf_distance(const DW& w, const Shape& a, const Shape& b) {
     if (a.kind == AVBD_SHAPE_HALFSPACE || b.kind == AVBD_SHAPE_HALFSPACE) return shape_distance(a, b, nullptr);
     const bool ta = a.kind == AVBD_SHAPE_HEIGHTFIELD, tb = b.kind == AVBD_SHAPE_HEIGHTFIELD;
     const bool ma = a.kind == AVBD_SHAPE_TRIMESH, mb = b.kind == AVBD_SHAPE_TRIMESH;
     // terrain against terrain or a mesh, mesh against mesh: separation
     if ((ta || ma) && (tb || mb)) return Dist{INFINITY, a.pos, b.pos};
-    if (ta) return hf_convex(w, a, b, true);
-    if (tb) return hf_convex(w, b, a, false);
-    if (ma) return mesh_convex(w, a, b, true);
-    if (mb) return mesh_convex(w, b, a, false);
+    if (ta) return hf_convex<WARP>(w, a, b, true);
+    if (tb) return hf_convex<WARP>(w, b, a, false);
+    if (ma) return mesh_convex<WARP>(w, a, b, true);
+    if (mb) return mesh_convex<WARP>(w, b, a, false);
     return shape_distance(a, b, nullptr);
 }
 // The rounded surface sits r closer along the witness axis; an infinite
@@ -231,19 +306,33 @@ static __device__ __forceinline__ Shape part_shape(const PartDesc& pt, V3 pos, Q
 }
 // compound_distance (distance.rs:550-599): the part reporting the smallest
 // distance, parts in order, each rounded part peeled inside its own query;
-// `first`: the compound owns pa.
+// `first`: the compound owns pa.  WARP: the parts over the lanes, or one by
+// one where each is itself a wide query.
+template <bool WARP>
 static __device__ __noinline__ Dist compound_distance(const DW& w, const Shape& c, const Shape& other, bool first) {
     const ExtDesc e = w.exts[(uint32_t)c.p.x];
     bool have = false;
     Dist best{INFINITY, c.pos, other.pos};
-    for (uint32_t k = 0; k < e.count; k++) {
+    auto query = [&](uint32_t k, auto wide) {
         const PartDesc pt = w.parts[e.first + k];
         const Shape child = part_shape(pt, c.pos + qrot(c.rot, ld3(pt.pos)), pose_world_rot(c.rot, ldq(pt.rot)));
-        Dist d = leaf_distance(w, child, other);
+        Dist d = leaf_distance<decltype(wide)::on>(w, child, other);
         if (pt.p.w > 0.0f) d = round_offset(d, pt.p.w, true, child.pos, other.pos);
-        if (!have || d.dist < best.dist) {
-            best = d;
-            have = true;
+        return d;
+    };
+    if (WARP && !wide_kind(other.kind)) {
+        Nearest near{best, 0xffffffffu};
+        for (uint32_t k = threadIdx.x & 31u; k < e.count; k += 32u) near.take(k, query(k, Wide<false>{}));
+        near.over_warp();
+        have = e.count > 0u;
+        best = near.best;
+    } else {
+        for (uint32_t k = 0; k < e.count; k++) {
+            const Dist d = query(k, Wide<WARP>{});
+            if (!have || d.dist < best.dist) {
+                best = d;
+                have = true;
+            }
         }
     }
     if (!have) return first ? Dist{INFINITY, c.pos, other.pos} : Dist{INFINITY, other.pos, c.pos};
@@ -252,6 +341,7 @@ static __device__ __noinline__ Dist compound_distance(const DW& w, const Shape& 
 // shape_distance with the wrapper arms (distance.rs:648-705): rounded shapes
 // peel first (a's, then b's), then compounds expand; compound against
 // compound is separation.  Rounded inners and compound parts are primitives.
+template <bool WARP>
 static __device__ __noinline__ Dist ext_distance_wrapped(const DW& w, const Shape& a, const Shape& b) {
     Shape ia = a, ib = b;
     float ra = 0.0f, rb = 0.0f;
@@ -267,18 +357,26 @@ static __device__ __noinline__ Dist ext_distance_wrapped(const DW& w, const Shap
     }
     Dist d;
     if (ia.kind == AVBD_SHAPE_COMPOUND && ib.kind == AVBD_SHAPE_COMPOUND) d = Dist{INFINITY, a.pos, b.pos};
-    else if (ia.kind == AVBD_SHAPE_COMPOUND) d = compound_distance(w, ia, ib, true);
-    else if (ib.kind == AVBD_SHAPE_COMPOUND) d = compound_distance(w, ib, ia, false);
-    else d = leaf_distance(w, ia, ib);
+    else if (ia.kind == AVBD_SHAPE_COMPOUND) d = compound_distance<WARP>(w, ia, ib, true);
+    else if (ib.kind == AVBD_SHAPE_COMPOUND) d = compound_distance<WARP>(w, ib, ia, false);
+    else d = leaf_distance<WARP>(w, ia, ib);
     if (b.kind == AVBD_SHAPE_ROUND) d = round_offset(d, rb, false, a.pos, b.pos);
     if (a.kind == AVBD_SHAPE_ROUND) d = round_offset(d, ra, true, a.pos, b.pos);
     return d;
 }
 // Primitive pairs keep the direct call; the wrapper arms take the rest.
+// WARP: every lane of a warp calls with the same pair, a wide one
+// (wide_pair).  A query is up to 0.1 ms of one thread, a body on terrain has
+// four to nine of them and a cast 24 times that: lists of wide pairs that
+// leave the chip idle (fits_warps) go a warp to a pair, longer ones a thread
+// to a pair, since most lanes of a warp have no query.  310 bodies of every
+// shape on terrain, a mesh and each other: a pass of two substeps 6.1 -> 3.8 ms.
+template <bool WARP = false>
 static __device__ __forceinline__ Dist ext_distance(const DW& w, const Shape& a, const Shape& b, float* sat_gap) {
     if (a.kind <= AVBD_SHAPE_HULL && b.kind <= AVBD_SHAPE_HULL) return shape_distance(a, b, sat_gap);
-    return ext_distance_wrapped(w, a, b);
+    return ext_distance_wrapped<WARP>(w, a, b);
 }
+static __device__ __forceinline__ bool fits_warps(uint32_t n) { return n <= gridDim.x * (blockDim.x / 32u); }
 // rows.rs:366-368
 static __device__ __forceinline__ bool pair_allowed(const DW& w, uint32_t a, uint32_t b) {
     uint2 fa = w.filter[a], fb = w.filter[b];

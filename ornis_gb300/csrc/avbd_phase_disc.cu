@@ -59,10 +59,12 @@ static __device__ __forceinline__ void discover_post(const DW& w, uint32_t a, ui
     r.separated = r.sgn > reach;
     r.keep = true;
 }
-// near_boxes (the filter): set, and nothing decided, for a new box pair whose
-// gap is within reach.
+// later (the filter): set, and nothing decided, for a new pair that a group
+// of lanes decides: 1 a box pair whose gap is within reach, 2 a wide pair.
+// WARP: every lane of a warp calls with the same wide pair.
+template <bool WARP>
 static __device__ __noinline__ Disc discover(const DW& w, uint32_t a, uint32_t b, bool need_witness,
-                                             bool* near_boxes = nullptr) {
+                                             int* later = nullptr) {
     Disc r;
     if (!discover_pre(w, a, b, r)) return r;
     if (r.exists && !need_witness) {
@@ -80,11 +82,15 @@ static __device__ __noinline__ Disc discover(const DW& w, uint32_t a, uint32_t b
         V3 nsat;
         float gap = separating_axis(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, nsat);
         float bound = GEN_MARGIN + len(ld3(w.vel[b]) - ld3(w.vel[a])) * w.dt * 1.00001f + 1e-6f;
-        if (near_boxes) *near_boxes = !(gap > bound);
+        if (later) *later = gap > bound ? 0 : 1;
+        return r;
+    }
+    if (later && wide_pair(sa.kind, sb.kind)) {
+        *later = 2;
         return r;
     }
     float sat = 0.0f;
-    r.d = ext_distance(w, sa, sb, &sat);
+    r.d = ext_distance<WARP>(w, sa, sb, &sat);
     r.sgn = boxes ? sat : r.d.dist;
     discover_post(w, a, b, sa, sb, r);
     return r;
@@ -112,9 +118,11 @@ static __device__ __forceinline__ void k_disc_filter_one(const DW& w, uint32_t c
         }
         return;
     }
-    bool box = false;
-    Disc d = discover(w, ab.x, ab.y, false, &box);
-    if (box) w.boxlist[agg_inc(&w.ctr[C_BOXNEW])] = c;  // k_disc_filter_boxes decides it
+    int later = 0;
+    Disc d = discover<false>(w, ab.x, ab.y, false, &later);
+    // k_disc_filter_boxes and k_disc_filter_wide decide these
+    if (later == 1) w.boxlist[agg_inc(&w.ctr[C_BOXNEW])] = c;
+    if (later == 2) w.boxlist[w.cand_cap - 1u - agg_inc(&w.ctr[C_WIDENEW])] = c;
     w.keep[c] = d.keep;
     if (d.keep) agg_inc_at(w.cnt, ab.x);
 }
@@ -133,6 +141,22 @@ __global__ void __launch_bounds__(128) k_disc_filter_boxes(DW w) {
         r.sgn = sat;
         discover_post(w, ab.x, ab.y, sa, sb, r);
         if ((threadIdx.x & 31u) == 0 && r.keep) {
+            w.keep[c] = 1;
+            atomicAdd(&w.cnt[ab.x], 1u);
+        }
+    }
+}
+__global__ void __launch_bounds__(128) k_disc_filter_wide(DW w) {
+    if (aborted(w)) return;
+    const uint32_t nw = w.ctr[C_WIDENEW];
+    const bool warp = fits_warps(nw);
+    const uint32_t per = warp ? 32u : 1u;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / per; i < nw; i += gridDim.x * blockDim.x / per) {
+        if (warp) __syncwarp();
+        const uint32_t c = w.boxlist[w.cand_cap - 1u - i];
+        const uint2 ab = w.cand[c];
+        const Disc r = warp ? discover<true>(w, ab.x, ab.y, false) : discover<false>(w, ab.x, ab.y, false);
+        if (r.keep && (!warp || (threadIdx.x & 31u) == 0)) {
             w.keep[c] = 1;
             atomicAdd(&w.cnt[ab.x], 1u);
         }
@@ -203,8 +227,10 @@ static __device__ __forceinline__ bool box_pair(const DW& w, uint2 ab) {
 // a warp run the same manifold code: corners of two boxes, of one, or none.
 static __device__ __forceinline__ void k_collect_boxes_one(const DW& w, uint32_t p) {
     uint2 ab = w.cand[w.slot_c[p]];
-    int boxes = (info_shape(w.info[ab.x]) == AVBD_SHAPE_BOX) + (info_shape(w.info[ab.y]) == AVBD_SHAPE_BOX);
-    if (boxes == 2) w.boxlist[agg_inc(&w.ctr[C_BOXPAIRS])] = p;
+    const uint32_t ka = info_shape(w.info[ab.x]), kb = info_shape(w.info[ab.y]);
+    int boxes = (ka == AVBD_SHAPE_BOX) + (kb == AVBD_SHAPE_BOX);
+    if (wide_pair(ka, kb)) w.clist[w.pair_cap - 1u - agg_inc(&w.ctr[C_WIDE])] = p;
+    else if (boxes == 2) w.boxlist[agg_inc(&w.ctr[C_BOXPAIRS])] = p;
     else if (boxes == 1) w.boxlist[w.pair_cap - 1u - agg_inc(&w.ctr[C_BOXONE])] = p;
     else w.clist[agg_inc(&w.ctr[C_NOBOX])] = p;
 }
@@ -243,7 +269,7 @@ static __device__ __forceinline__ void k_disc_build_one(const DW& w, uint32_t p)
         build_pair(w, p, ab, r);
         return;
     }
-    build_pair(w, p, ab, discover(w, ab.x, ab.y, true));
+    build_pair(w, p, ab, discover<false>(w, ab.x, ab.y, true));
 }
 static __device__ __forceinline__ void build_pair(const DW& w, uint32_t p, uint2 ab, const Disc& d) {
     uint32_t ia = ab.x, ib = ab.y;
@@ -393,6 +419,19 @@ __global__ void __launch_bounds__(128, 4) k_disc_build(DW w) {
         k_disc_build_one(w, p);
     }
 }
+__global__ void __launch_bounds__(128, 4) k_disc_build_wide(DW w) {
+    if (aborted(w)) return;
+    const uint32_t n = w.ctr[C_WIDE];
+    const bool warp = fits_warps(n);
+    const uint32_t per = warp ? 32u : 1u;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / per; i < n; i += gridDim.x * blockDim.x / per) {
+        if (warp) __syncwarp();
+        const uint32_t p = w.clist[w.pair_cap - 1u - i];
+        const uint2 ab = w.cand[w.slot_c[p]];
+        const Disc r = warp ? discover<true>(w, ab.x, ab.y, true) : discover<false>(w, ab.x, ab.y, true);
+        if (!warp || (threadIdx.x & 31u) == 0) build_pair(w, p, ab, r);
+    }
+}
 
 // Long static segments, in (b, candidate) order: every chunk of SORT_CHUNK
 // slots is sorted in shared memory (bitonic network), then each slot's final
@@ -464,6 +503,7 @@ __global__ void k_sort_long_rank(DW w) {
 void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int triggers) {
     k_disc_filter<<<gsz(w.cand_cap, 128), 128, 0, st>>>(w, triggers && w.evs ? 1 : 0);
     k_disc_filter_boxes<<<gsz(w.cand_cap, 4), 128, 0, st>>>(w);
+    if (wide_world(w)) k_disc_filter_wide<<<gsz(w.cand_cap, 4), 128, 0, st>>>(w);
     scan_exclusive(w.cnt, w.offA, w.N + 1, scan_tmp, st);
     k_place<<<gsz(w.cand_cap, 256), 256, 0, st>>>(w);
     k_sort_slots<<<nblk(w.N, 256), 256, 0, st>>>(w);
@@ -474,6 +514,7 @@ void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int trig
     k_collect_boxes<<<gsz(w.pair_cap, 256), 256, 0, st>>>(w);
     k_box_witness<<<gsz(w.pair_cap, 4), 128, 0, st>>>(w);
     k_disc_build<<<dim3(gsz(w.pair_cap, 128), 3), 128, 0, st>>>(w);
+    if (wide_world(w)) k_disc_build_wide<<<gsz(w.pair_cap, 32), 128, 0, st>>>(w);
 }
 
 // ---- after discovery ----------------------------------------------------------

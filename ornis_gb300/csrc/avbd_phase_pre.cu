@@ -274,7 +274,7 @@ __global__ void k_prologue(DW w) {
     uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h == 0) {
         const int zero[] = {C_CCD_PENDING, C_BOXPAIRS, C_FCAND, C_BOXONE, C_NOBOX, C_LONGSEG, C_CAND, C_NCOL, C_FAST,
-                            C_POINTS, C_SLEEP, C_CCD_HITS, C_ROLL, C_BOXNEW, C_FBOX, C_GBAR, C_CBAR, C_LBAR, C_COLPEND, C_COLPEND + 1, C_COLPEND + 2, C_COLPEND + 3};
+                            C_POINTS, C_SLEEP, C_CCD_HITS, C_ROLL, C_BOXNEW, C_FBOX, C_WIDENEW, C_WIDE, C_GBAR, C_CBAR, C_LBAR, C_COLPEND, C_COLPEND + 1, C_COLPEND + 2, C_COLPEND + 3};
         for (int k : zero) w.ctr[k] = 0;
         if (w.evs) w.evs[EV_TRIG_NOW] = 0;
     }
@@ -791,8 +791,9 @@ struct Cast {
     V3 normal;
     V3 point;  // the target's witness at the hit
 };
-// WARP: a box against a box, every lane of a warp calling with the same bodies.
-template <bool WARP>
+// WARP: a box against a box or (WIDE) a wide pair, every lane of a warp
+// calling with the same bodies.
+template <bool WARP, bool WIDE>
 static __device__ __noinline__ Cast cast_one(const DW& w, uint32_t h, uint32_t o) {
     Cast c{false, 0.0f, V0(), V0()};
     V3 disp = ld3(w.vel[h]) * w.dt;
@@ -805,7 +806,11 @@ static __device__ __noinline__ Cast cast_one(const DW& w, uint32_t h, uint32_t o
     float t = 0.0f;
     for (int it = 0; it < 24; it++) {
         mv.pos = p0 + dir * t;
-        const Dist d = WARP ? box_box_warp(mv.pos, mv.rot, mv.p, tg.pos, tg.rot, tg.p, nullptr) : ext_distance(w, mv, tg, nullptr);
+        Dist d;
+        if (WARP && (!WIDE || (mv.kind == AVBD_SHAPE_BOX && tg.kind == AVBD_SHAPE_BOX)))
+            d = box_box_warp(mv.pos, mv.rot, mv.p, tg.pos, tg.rot, tg.p, nullptr);
+        else
+            d = ext_distance<WARP>(w, mv, tg, nullptr);
         if (d.dist <= SHAPE_TOUCH) {
             if (t > 0.0f) {
                 c.hit = true;
@@ -852,7 +857,7 @@ static __device__ __forceinline__ bool sweep_may_touch(const DW& w, uint32_t h, 
 // casting again: the winner's inputs do not change between its cast and its
 // apply (a mover applies once its earlier movers are final and it has recast
 // against any that moved; later movers wait for it).
-template <bool WARP>
+template <bool WARP, bool WIDE>
 static __device__ __forceinline__ void k_ccd_cast_one(const DW& w, int first, uint32_t c, uint32_t tag) {
     uint2 ab = w.cand[c];
     bool fa = w.fast[ab.x], fb = w.fast[ab.y];
@@ -863,7 +868,7 @@ static __device__ __forceinline__ void k_ccd_cast_one(const DW& w, int first, ui
         if (!first && !(w.ccd_state[h] == 0 && w.ccd_deps[h] == 0 && w.ccd_recompute[h] == 1)) continue;
         if (!ccd_target(w, h, o)) continue;
         if (!sweep_may_touch(w, h, o)) continue;
-        Cast r = cast_one<WARP>(w, h, o);
+        Cast r = cast_one<WARP, WIDE>(w, h, o);
         if (r.hit && (!WARP || (threadIdx.x & 31u) == 0)) {
             // earliest time wins; equal times keep the lower handle (distance.rs:886-890)
             unsigned long long key = ((unsigned long long)__float_as_uint(r.t) << 32) | o;
@@ -891,20 +896,35 @@ __global__ void k_ccd_collect(DW w) {
         uint2 ab = w.cand[c];
         bool fa = w.fast[ab.x], fb = w.fast[ab.y];
         if (!fa && !fb) continue;
-        if (info_shape(w.info[ab.x]) == AVBD_SHAPE_BOX && info_shape(w.info[ab.y]) == AVBD_SHAPE_BOX)
+        const uint32_t ka = info_shape(w.info[ab.x]), kb = info_shape(w.info[ab.y]);
+        if ((ka == AVBD_SHAPE_BOX && kb == AVBD_SHAPE_BOX) || wide_pair(ka, kb))
             w.fcand[w.cand_cap - 1u - agg_inc(&w.ctr[C_FBOX])] = c;
         else
             w.fcand[agg_inc(&w.ctr[C_FCAND])] = c;
         if (fa && fb && ccd_target(w, ab.x, ab.y)) atomicAdd(&w.ccd_deps[ab.y], 1u);
     }
 }
+template <bool WIDE>
 static __device__ __forceinline__ void ccd_cast_all(const DW& w, int first, uint32_t tag) {
-    // box pairs a warp each (a cast is up to 24 distance queries in a row), the rest a thread each
+    // box pairs a warp each (a cast is up to 24 distance queries in a row),
+    // wide pairs too while the list is short, the rest a thread each
     const uint32_t n = w.ctr[C_FCAND], nb = w.ctr[C_FBOX], warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nb; i += warps)
-        k_ccd_cast_one<true>(w, first, w.fcand[w.cand_cap - 1u - i], tag);
+    const bool wide = !WIDE || fits_warps(nb);
+    auto is_wide = [&](uint32_t c) {
+        return wide_pair(info_shape(w.info[w.cand[c].x]), info_shape(w.info[w.cand[c].y]));
+    };
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nb; i += warps) {
+        __syncwarp();
+        const uint32_t c = w.fcand[w.cand_cap - 1u - i];
+        if (wide || !is_wide(c)) k_ccd_cast_one<true, WIDE>(w, first, c, tag);
+    }
+    if (!wide)
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x) {
+            const uint32_t c = w.fcand[w.cand_cap - 1u - i];
+            if (is_wide(c)) k_ccd_cast_one<false, WIDE>(w, first, c, tag);
+        }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        k_ccd_cast_one<false>(w, first, w.fcand[i], tag);
+        k_ccd_cast_one<false, WIDE>(w, first, w.fcand[i], tag);
 }
 // The record of each mover's winning cast of round `tag` (the one whose key
 // equals the mover's best; keys are unique per mover).
@@ -932,7 +952,7 @@ static __device__ void ccd_apply(const DW& w, uint32_t h, bool recorded) {
             const float4* rec = w.ccd_hit + (size_t)k * 3;
             r = Cast{true, rec[0].x, ld3(rec[1]), ld3(rec[2])};
         } else {
-            r = cast_one<false>(w, h, o);  // the winning cast again: same inputs, same t and normal
+            r = cast_one<false, false>(w, h, o);  // the winning cast again: same inputs, same t and normal
         }
         V3 disp = ld3(w.vel[h]) * w.dt;
         float L = fmaxf(len(disp), MIN_TOI_DISP_LENGTH);
@@ -992,6 +1012,9 @@ static __device__ __forceinline__ bool ccd_recasts(const DW& w, uint32_t h) {
 // the phases of a round; a substep ends at the round that settles its last
 // mover (at once without any), where a launch per phase ran all 42 of them
 // (0.17 ms with nothing to cast).
+// WIDE: the world has terrain, meshes or compounds (the rest is not slowed by
+// the registers and stack of their queries over a warp: 1.2x on 100,000 bodies).
+template <bool WIDE>
 __global__ void __launch_bounds__(128) k_ccd_rounds(DW w, int sync) {
     if (aborted(w) || w.ctr[C_FAST] == 0u) return;
     __shared__ uint32_t s_ok;
@@ -999,7 +1022,7 @@ __global__ void __launch_bounds__(128) k_ccd_rounds(DW w, int sync) {
     uint32_t target = 0;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
     const uint32_t nfast = w.ctr[C_FAST];
-    ccd_cast_all(w, 1, 0u);
+    ccd_cast_all<WIDE>(w, 1, 0u);
     if (!all_sync(w, bar, sync, target, &s_ok)) return;
     ccd_pick(w, 0u);
     if (!all_sync(w, bar, sync, target, &s_ok)) return;
@@ -1022,7 +1045,7 @@ __global__ void __launch_bounds__(128) k_ccd_rounds(DW w, int sync) {
             if (w.ccd_win) w.ccd_win[h] = ~0u;
         }
         if (!all_sync(w, bar, sync, target, &s_ok)) return;
-        ccd_cast_all(w, 0, (uint32_t)(r + 1));
+        ccd_cast_all<WIDE>(w, 0, (uint32_t)(r + 1));
         if (!all_sync(w, bar, sync, target, &s_ok)) return;
         ccd_pick(w, (uint32_t)(r + 1));
         if (!all_sync(w, bar, sync, target, &s_ok)) return;
@@ -1031,8 +1054,11 @@ __global__ void __launch_bounds__(128) k_ccd_rounds(DW w, int sync) {
 void launch_ccd(const DW& w, cudaStream_t st) {
     if (!w.enable_ccd) return;
     k_ccd_collect<<<gsz(w.cand_cap, 256), 256, 0, st>>>(w);
-    static Resident r;
-    launch_synced(r, k_ccd_rounds, 128, 0, w.N, st, w);
+    static Resident r, rw;
+    // a wide world's casts take up to 1 ms: a block per two bodies, where the
+    // others' small worlds gain more from a cluster's shorter start
+    if (wide_world(w)) launch_synced(rw, k_ccd_rounds<true>, 128, 0, 8 * (int)w.N, st, w);
+    else launch_synced(r, k_ccd_rounds<false>, 128, 0, w.N, st, w);
 }
 
 }  // namespace avbd

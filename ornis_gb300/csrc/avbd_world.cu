@@ -589,6 +589,7 @@ static int upload_all(AvbdWorld* W) {
     DW& w = W->w;
     cudaStream_t st = W->st;
     // convex hull tables (rebuilt on every full upload: hulls are few and small)
+    const DW before = w;
     W->hullmem.release();
     w.hulls = nullptr;
     w.nhulls = 0;
@@ -701,6 +702,10 @@ static int upload_all(AvbdWorld* W) {
         w.meshes = dd;
         w.nmeshes = (uint32_t)md.size();
     }
+    // captured launches hold the tables, and which kernels a wide world runs
+    if (before.hulls != w.hulls || before.exts != w.exts || before.parts != w.parts || before.hfs != w.hfs ||
+        before.meshes != w.meshes || before.nhulls != w.nhulls || wide_world(before) != wide_world(w))
+        free_graphs(W);
     for (uint32_t h = 0; h < N; h++) {
         const AvbdBody& b = W->bodies[h];
         if (b.shape > AVBD_SHAPE_TRIMESH) return AVBD_ERR_UNSUPPORTED;

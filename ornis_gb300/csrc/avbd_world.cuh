@@ -81,11 +81,13 @@ enum Ctr {
     C_CCD_HITS = 18,     // swept-cast hits recorded this substep (ccd_hit)
     C_ROLL = 19,         // a touching pair has rolling or torsion friction (k_entries)
     C_BOXNEW = 20,       // new box-box candidates near enough for the witness test
-    C_FBOX = 21,         // candidates with a fast body that are box pairs (listed from the back of fcand)
+    C_FBOX = 21,         // candidates with a fast body that are box or wide pairs (listed from the back of fcand)
     C_CBAR = 22,         // arrivals at the grid barrier of the swept casts, this substep
     C_LBAR = 23,         // arrivals at the grid barrier of the large scenes' colouring, this substep
     C_COLPEND = 24,      // four words: a body is uncoloured after round r (word r mod 4)
-    C_NUM = 28
+    C_WIDENEW = 28,      // new wide candidates (from the back of boxlist, until the filter is done)
+    C_WIDE = 29,         // wide pairs: terrain, meshes, compounds (from the back of clist)
+    C_NUM = 30
 };
 enum ErrBits { E_CAND_OVERFLOW = 1, E_COLOUR_OVERFLOW = 2, E_TIMEOUT = 4, E_COLOUR_RANGE = 8 };
 
@@ -265,7 +267,7 @@ struct DW {
     uint32_t* long_seg;            // N: static bodies with a long pair segment (C_LONGSEG of them)
     unsigned long long* seg_key;  // cand_cap: (b, candidate) keys of those segments, sorted per chunk
     uint32_t* boxlist; // box-box pair slots from the front, one-box pair slots from the back
-    uint32_t* clist;   // pair slots without a box
+    uint32_t* clist;   // slots of pairs without a box from the front, of wide pairs from the back
     float4 *bd_pa, *bd_pb;  // box-box witnesses per pair slot: (pa, dist), (pb, SAT gap)
     float4* p_t1;           // first tangent of every pair's friction frame (takes over bd_pa as each pair is built)
     float4 *aabb_lo, *aabb_hi;
@@ -274,7 +276,7 @@ struct DW {
 
     // CCD scratch
     uint32_t* fbody;  // N: the fast bodies of this substep (C_FAST of them)
-    uint32_t* fcand;  // cand_cap: candidates with a fast body: C_FCAND from the front, C_FBOX box pairs from the back
+    uint32_t* fcand;  // cand_cap: candidates with a fast body: C_FCAND from the front, C_FBOX box and wide pairs from the back
     uint8_t* fast;
     unsigned long long* ccd_best;
     uint32_t* ccd_deps;
@@ -319,6 +321,8 @@ struct DW {
     uint32_t *col_key, *col_key2, *col_val, *col_hist;
     uint32_t* ctr;       // counters
 };
+// The world may hold terrain, meshes or compounds (wide pairs).
+static inline bool wide_world(const DW& w) { return w.nexts || w.nhfs || w.nmeshes; }
 
 // One recomputed substep as the adjoint kernels read it: the frozen contact
 // set and colouring, the step-start and target poses, and the iterates.
