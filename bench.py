@@ -480,7 +480,7 @@ def oracle_parity(w, offs, params, nsub, nscenes=8, steps=3, split=True, threads
     current state, for `steps` steps.  Before every substep, each sampled
     scene's state is exported from the device and loaded into an f32 and an
     f64 oracle world (Coloured order; rows summed per pair when the device
-    runs the split or per-scene launch); the device steps the whole batch one
+    does); the device steps the whole batch one
     substep (the reference's step_inner) in the benchmarked configuration
     and the oracles step their scene.  Integer outputs (pair sets, points per
     pair, contact IDs, colours) are compared exactly; poses relative to
@@ -804,7 +804,7 @@ def adjoint_rate(args):
     w.set_events(-1)
     s0 = w.export_state()
     fwd = {}
-    for lanes in (1, 0):  # thread-per-body primal, then the split primal the rollout runs
+    for lanes in (1, 0):  # rows in the reference's order ("thread"), then per pair ("split"), which the rollout runs
         w.set_tuning(lanes, 128)
         w.step_graph(nsub * 3)  # warm-up: graphs captured
         w.import_state(s0)
@@ -853,7 +853,7 @@ def adjoint_rate(args):
             "cpu_baseline": cpu,
             "how": "wall time with the host waiting; backward = per-segment recompute from the checkpoint "
                    "plus the reverse sweep; forward = the same rollout by CUDA-graph replay with the faster "
-                   "of the two primal launches (the rollout itself runs the split primal); the second of two "
+                   "of the two row orders (the rollout itself adds rows up per pair); the second of two "
                    "rollouts from the same start is timed (the first sets up the frames and recording graphs, "
                    "as the forward's warm-up captures its graphs)"}
 

@@ -532,15 +532,15 @@ int avbd_world_get_colours(AvbdWorld* world, int32_t* colours, uint32_t n);
  * a half-space must be static. */
 int avbd_body_init(AvbdBody* out, uint32_t shape, const float* params, const float* position, float mass);
 
-/* Launch shape of the primal kernel: lanes cooperating on one body (1, 4, 8,
- * 16 or 32) and threads per block; 0 = the split launch (per colour, one
- * thread per (pair, side) for the rows, then one per body for the sums and
- * the solve); AVBD_PRIMAL_SCENES = the per-scene solve (one block takes a
- * scene through every iteration of a substep — all colours' primal and the
- * dual — in one launch per substep; block 128, 256 or 512; the split
- * arithmetic; a world with a scene above 2048 bodies runs the split launches
- * instead).  No reference counterpart (the reference sweeps on one CPU
- * thread); picked by the autotuner in ornis_gb300/tune.py. */
+/* Form of the iterations.  1 (default), 0 and AVBD_PRIMAL_SCENES: every
+ * iteration of a substep — all colours' primal and the dual — in one launch,
+ * a warp per tile of up to 32 bodies; 1 adds a body's rows up in the
+ * reference's order, 0 and AVBD_PRIMAL_SCENES per pair first.  4, 8, 16 or
+ * 32: that many lanes cooperating on one body, a launch per colour.
+ * primal_block: threads per block of the lanes form (the one-launch forms
+ * choose their own; its value is checked as before).  No reference
+ * counterpart (the reference sweeps on one CPU thread); picked by the
+ * autotuner in ornis_gb300/tune.py. */
 #define AVBD_PRIMAL_SCENES (-1)
 int avbd_set_tuning(AvbdWorld* world, int primal_lanes, int primal_block);
 
@@ -555,16 +555,16 @@ int avbd_set_tuning(AvbdWorld* world, int primal_lanes, int primal_block);
  * both. */
 int avbd_set_precision(AvbdWorld* world, int fast);
 
-/* Register budget of the one-thread-per-body primal: built for 4, 6 or 8
- * resident 128-thread blocks per SM.  Picked by the autotuner. */
+/* A hint of earlier launch forms (resident 128-thread blocks per SM: 4, 6 or
+ * 8), checked and kept; the one-launch iterations choose their own. */
 int avbd_set_occupancy(AvbdWorld* world, int min_blocks);
 
 /* Start (on != 0) or stop profiler collection (cudaProfilerStart/Stop). */
 int avbd_profiler(int on);
 
-/* Order of the bodies inside each colour's launch: 0 = ascending handle,
- * 1 = by incident-pair count (less warp divergence).  Results do not depend
- * on it: bodies of one colour are independent. */
+/* Order of the bodies inside each colour: 0 = ascending handle, 1 = by
+ * incident-pair count.  A hint: the tiles take either, and results do not
+ * depend on it (bodies of one colour are independent). */
 int avbd_set_work_order(AvbdWorld* world, int by_work);
 
 /* Scenes of at most `small_scene_max` bodies (0..2048, default 2048) are
@@ -677,7 +677,7 @@ int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* bodies, uin
  * avbd_world_step_graph) and keep a device checkpoint of the full step
  * state every `checkpoint_every` steps, for avbd_adjoint_backward.  Worlds
  * with rolling / torsion friction, motors, or joints other than Ball and
- * Revolute return AVBD_ERR_UNSUPPORTED.  The rollout runs the split primal launch
+ * Revolute return AVBD_ERR_UNSUPPORTED.  The rollout adds rows up per pair
  * (avbd_set_tuning lanes 0) and orders every body's contact pairs (the
  * static bodies' too), which the world keeps afterwards; retuning the
  * world before the backward invalidates the recording.  A new forward

@@ -66,7 +66,7 @@ AXIS_LIMITED = 2
 
 MAX_POINTS = 8
 
-# avbd_set_tuning lanes value of the per-scene solve (one block per scene)
+# avbd_set_tuning lanes value of the one-launch iterations with rows added up per pair (as 0)
 PRIMAL_SCENES = -1
 
 F3 = C.c_float * 3
