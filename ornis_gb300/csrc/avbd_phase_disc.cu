@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(128) k_disc_filter_wide(DW w) {
 __global__ void __launch_bounds__(128, 4) k_disc_filter(DW w, int triggers) {
     if (aborted(w)) return;
     const uint32_t n = n_cand(w);
-    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
-        k_disc_filter_one(w, c, triggers);
+    const Spread sp = spread_entries(w, n);
+    for (uint32_t c = sp.first; c < n; c += sp.step) k_disc_filter_one(w, c, triggers);
 }
 
 static __device__ __forceinline__ void k_place_one(const DW& w, uint32_t c) {
@@ -414,7 +414,8 @@ __global__ void __launch_bounds__(128, 4) k_disc_build(DW w) {
     if (aborted(w)) return;
     const int cls = (int)blockIdx.y;
     const uint32_t n = w.ctr[cls == 0 ? C_BOXPAIRS : (cls == 1 ? C_BOXONE : C_NOBOX)];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const Spread sp = spread_entries(w, n);
+    for (uint32_t i = sp.first; i < n; i += sp.step) {
         uint32_t p = cls == 0 ? w.boxlist[i] : (cls == 1 ? w.boxlist[w.pair_cap - 1u - i] : w.clist[i]);
         k_disc_build_one(w, p);
     }
@@ -501,7 +502,8 @@ __global__ void k_sort_long_rank(DW w) {
 }
 
 void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int triggers) {
-    k_disc_filter<<<gsz(w.cand_cap, 128), 128, 0, st>>>(w, triggers && w.evs ? 1 : 0);
+    const int per = mixed_world(w) ? 32 : 128;  // room for spread_entries
+    k_disc_filter<<<gsz(w.cand_cap, per), 128, 0, st>>>(w, triggers && w.evs ? 1 : 0);
     k_disc_filter_boxes<<<gsz(w.cand_cap, 4), 128, 0, st>>>(w);
     if (wide_world(w)) k_disc_filter_wide<<<gsz(w.cand_cap, 4), 128, 0, st>>>(w);
     scan_exclusive(w.cnt, w.offA, w.N + 1, scan_tmp, st);
@@ -513,7 +515,7 @@ void launch_discovery(const DW& w, uint32_t* scan_tmp, cudaStream_t st, int trig
     }
     k_collect_boxes<<<gsz(w.pair_cap, 256), 256, 0, st>>>(w);
     k_box_witness<<<gsz(w.pair_cap, 4), 128, 0, st>>>(w);
-    k_disc_build<<<dim3(gsz(w.pair_cap, 128), 3), 128, 0, st>>>(w);
+    k_disc_build<<<dim3(gsz(w.pair_cap, per), 3), 128, 0, st>>>(w);
     if (wide_world(w)) k_disc_build_wide<<<gsz(w.pair_cap, 32), 128, 0, st>>>(w);
 }
 

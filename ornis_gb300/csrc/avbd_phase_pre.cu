@@ -923,8 +923,8 @@ static __device__ __forceinline__ void ccd_cast_all(const DW& w, int first, uint
             const uint32_t c = w.fcand[w.cand_cap - 1u - i];
             if (is_wide(c)) k_ccd_cast_one<false, WIDE>(w, first, c, tag);
         }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        k_ccd_cast_one<false, WIDE>(w, first, w.fcand[i], tag);
+    const Spread sp = spread_entries(w, n);
+    for (uint32_t i = sp.first; i < n; i += sp.step) k_ccd_cast_one<false, WIDE>(w, first, w.fcand[i], tag);
 }
 // The record of each mover's winning cast of round `tag` (the one whose key
 // equals the mover's best; keys are unique per mover).

@@ -321,7 +321,9 @@ struct DW {
     uint32_t *col_key, *col_key2, *col_val, *col_hist;
     uint32_t* ctr;       // counters
 };
-// The world may hold terrain, meshes or compounds (wide pairs).
+// The world may hold shapes whose queries are long and unlike.
+__host__ __device__ inline bool mixed_world(const DW& w) { return w.nhulls || w.nexts || w.nhfs || w.nmeshes; }
+// It may hold terrain, meshes or compounds (wide pairs).
 static inline bool wide_world(const DW& w) { return w.nexts || w.nhfs || w.nmeshes; }
 
 // One recomputed substep as the adjoint kernels read it: the frozen contact
