@@ -39,7 +39,10 @@ extern "C" {
 #define AVBD_ERR_INVALID_ARG (-1)    /* null pointer, bad size, bad enum       */
 #define AVBD_ERR_CAPACITY (-2)       /* a device buffer would overflow         */
 #define AVBD_ERR_DEVICE (-3)         /* a CUDA call failed                     */
-#define AVBD_ERR_TIMEOUT (-4)        /* a bounded device wait gave up          */
+#define AVBD_ERR_TIMEOUT (-4)        /* a bounded device wait gave up: the world
+                                        is between steps; it can be read, but
+                                        steps and snapshots return this until a
+                                        whole state is imported                */
 #define AVBD_ERR_NONFINITE (-5)      /* NaN/Inf in an input body               */
 #define AVBD_ERR_UNSUPPORTED (-6)    /* shape / joint kind not implemented     */
 #define AVBD_ERR_FORMAT (-7)         /* not a snapshot of this format version,

@@ -420,12 +420,16 @@ static __device__ __forceinline__ void wake_body(const DW& w, uint32_t h) {
 }
 // A candidate-buffer overflow aborts the rest of the substep (every later
 // kernel returns at once) so the host can grow the buffers and replay it: the
-// kernels that ran before the check (wake, torque, AABBs) are idempotent.
-static __device__ __forceinline__ bool aborted(const DW& w) { return (w.ctr[C_ERR] & E_CAND_OVERFLOW) != 0u; }
+// kernels that ran before the check (wake, torque, AABBs) are idempotent.  A
+// grid barrier that gave up aborts it too: nothing is built on what its
+// launch left unfinished.
+static __device__ __forceinline__ bool aborted(const DW& w) {
+    return (w.ctr[C_ERR] & (E_CAND_OVERFLOW | E_TIMEOUT)) != 0u;
+}
 // The iterations of a substep whose colouring needs more colours than the
 // launched iteration covers are skipped; the host finishes that substep.
 static __device__ __forceinline__ bool aborted_solve(const DW& w) {
-    return (w.ctr[C_ERR] & (E_CAND_OVERFLOW | E_COLOUR_RANGE)) != 0u;
+    return (w.ctr[C_ERR] & (E_CAND_OVERFLOW | E_TIMEOUT | E_COLOUR_RANGE)) != 0u;
 }
 static __device__ __forceinline__ uint32_t n_cand(const DW& w) { return min(w.ctr[C_CAND], w.cand_cap); }
 static __device__ __forceinline__ uint32_t n_pairs(const DW& w) { return w.offA[w.N]; }
@@ -609,10 +613,11 @@ static __device__ __forceinline__ bool joint_driven(const DW& w, uint32_t j) {
 // Barrier over a launch's blocks, all of them resident: one block, a cluster
 // (the hardware's barrier, about 0.3 us), or a cooperative grid (about 1.5
 // us).  The grid's counts arrivals in *bar, a counter that k_prologue zeroes,
-// and gives up after a bounded number of polls: the error bit then reaches
-// the host.  A block may work between its arrival and its wait.
+// and gives up after w.polls polls (GRID_POLLS: some seconds): its block
+// returns, the others' polls run out in turn, later kernels of the substep
+// return at once, and the error bit reaches the host.  A block may work
+// between its arrival and its wait.
 enum SyncKind { SYNC_BLOCK = 0, SYNC_CLUSTER = 1, SYNC_GRID = 2 };
-constexpr uint32_t GRID_POLLS = 1u << 23;
 static __device__ __forceinline__ void all_arrive(uint32_t* bar, int kind) {
     if (kind == SYNC_CLUSTER) {
         asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -637,8 +642,8 @@ static __device__ __forceinline__ bool all_wait(const DW& w, uint32_t* bar, int 
     if (threadIdx.x == 0) {
         uint32_t good = 1u, n = 0u;
         while (*reinterpret_cast<volatile uint32_t*>(bar) < target)
-            if (++n > GRID_POLLS) {
-                atomicOr(&w.ctr[C_ERR], (uint32_t)E_TIMEOUT);
+            if (++n > w.polls) {
+                if (!(atomicOr(&w.ctr[C_ERR], (uint32_t)E_TIMEOUT) & E_TIMEOUT)) atomicAdd(&w.ctr[C_TIMEOUT], 1u);
                 good = 0u;
                 break;
             }

@@ -587,7 +587,7 @@ __device__ __forceinline__ uint32_t row_lower(const uint32_t* keys, uint32_t lo,
 constexpr uint32_t ROW_SKIP = 16;  // bodies of one key passed over one by one
 __global__ void k_sap_row_sweep(DW w, uint32_t b0, uint32_t n, const float* ext, const uint32_t* row_key) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= n || aborted(w)) return;
     const uint32_t a = w.sort_idx[i], rk = row_key[a - b0];
     if (rk == 0xffffffffu) return;  // a half-space
     const float4 alo = w.aabb_lo[a], ahi = w.aabb_hi[a];
@@ -646,6 +646,7 @@ struct SortBufs {
 };
 __global__ void __launch_bounds__(256) k_sap_sort(DW w, SortBufs sb, uint32_t b0, uint32_t n, uint32_t rounds, uint32_t* bar,
                                                   int sync) {
+    if (aborted(w)) return;
     __shared__ uint32_t base[256], cnt[8][256], wsum[8], s_ok;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, ntiles = gridDim.x;
     const uint32_t first = blockIdx.x * rounds * 256u;

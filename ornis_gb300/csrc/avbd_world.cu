@@ -263,6 +263,8 @@ struct AvbdWorld {
     size_t graph_nodes = 0;       // kernel nodes in one captured substep (no events)
     size_t graph_nodes_emit = 0;  // ... in one that reports events
     uint64_t steps = 0;
+    uint32_t polls = GRID_POLLS;
+    bool half_stepped = false;  // a substep was cut short: no steps until a state is imported
     AdjTape* adj = nullptr;  // checkpoints of the last differentiable rollout
     uint64_t mem_gen = 0;    // bumped whenever the device arrays are (re)allocated or a launch setting changes
 };
@@ -507,6 +509,7 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     w.enable_sleep = W->prm.enable_sleep;
     w.enable_ccd = W->prm.enable_ccd;
     w.max_cols = MAX_COLOURS;
+    w.polls = W->polls;
     set_pair_ptrs(W);
     return AVBD_OK;
 }
@@ -1191,9 +1194,11 @@ static void accumulate(AvbdWorld* W) {
     W->cum.timeouts = c[C_TIMEOUT] + c[C_CCD_LEFT];
 }
 
-// A grid barrier of the iterations gave up: the substep is not complete.
+// A grid barrier gave up: the substep is not complete.
 static int timed_out(AvbdWorld* W) {
     if (!(W->h_ctr[C_ERR] & E_TIMEOUT)) return AVBD_OK;
+    W->half_stepped = true;
+    W->cum.timeouts = W->h_ctr[C_TIMEOUT] + W->h_ctr[C_CCD_LEFT];
     CK(cudaMemsetAsync(W->w.ctr + C_ERR, 0, 4, W->st));
     return AVBD_ERR_TIMEOUT;
 }
@@ -1225,9 +1230,10 @@ static int substep_plain(AvbdWorld* W, bool emit) {
             rc = read_ctr(W);
             if (rc) return rc;
         }
+        rc = timed_out(W);
+        if (rc) return rc;
         accumulate(W);
-        if (W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW) return AVBD_ERR_CAPACITY;
-        return timed_out(W);
+        return W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW ? AVBD_ERR_CAPACITY : AVBD_OK;
     }
     return AVBD_ERR_CAPACITY;
 }
@@ -1546,9 +1552,10 @@ int adj_substep(AvbdWorld* W, AdjTape* t, int k) {
             W->last_ncol = (int)ncol;
             f.npairs = P;
             f.ncol = ncol;
+            const int late = timed_out(W);
+            if (late) return late;
             accumulate(W);
-            if (W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW) return AVBD_ERR_CAPACITY;
-            return timed_out(W);
+            return W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW ? AVBD_ERR_CAPACITY : AVBD_OK;
         }
         // candidate overflow: nothing after the broadphase ran; undo the flip
         // and record this substep plainly after growing
@@ -1581,9 +1588,10 @@ int adj_substep(AvbdWorld* W, AdjTape* t, int k) {
     CK(cudaGetLastError());
     int rc = read_ctr(W);
     if (rc) return rc;
+    rc = timed_out(W);
+    if (rc) return rc;
     accumulate(W);
-    if (W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW) return AVBD_ERR_CAPACITY;
-    return timed_out(W);
+    return W->h_ctr[C_ERR] & E_COLOUR_OVERFLOW ? AVBD_ERR_CAPACITY : AVBD_OK;
 }
 
 int adj_reverse(AvbdWorld* W, AdjTape* t, const AdjFrame& f) {
@@ -2397,6 +2405,7 @@ int avbd_world_sync(AvbdWorld* W) {
 }
 
 static int begin_steps(AvbdWorld* W) {
+    if (W->half_stepped) return AVBD_ERR_TIMEOUT;
     cudaSetDevice(W->device);
     if (W->host_valid && W->dev_valid) {
         W->host_valid = false;
@@ -2527,9 +2536,9 @@ static int step_graph_n(AvbdWorld* W, int32_t substeps, bool last_only) {
             rc = read_ctr(W);
             if (rc) return rc;
         }
-        accumulate(W);
         rc = timed_out(W);
         if (rc) return rc;
+        accumulate(W);
     }
     return AVBD_OK;
 }
@@ -2597,6 +2606,7 @@ int avbd_world_import_state(AvbdWorld* W, const AvbdBody* bodies, const AvbdBody
     }
     if (joints)
         for (size_t i = 0; i < W->joints.size(); i++) W->joints[i].st = joints[i];
+    if (bodies && aux && pairs && (joints || W->joints.empty())) W->half_stepped = false;  // a whole state
     W->time_debt = 0.0f;
     return AVBD_OK;
 }
@@ -2691,6 +2701,14 @@ int avbd_set_tuning(AvbdWorld* W, int primal_lanes, int primal_block) {
 int avbd_set_joint_stiffness(AvbdWorld* W, float k) {
     if (!W || !std::isfinite(k) || k < 0.0f) return AVBD_ERR_INVALID_ARG;
     W->w.joint_k = k;
+    free_graphs(W);
+    return AVBD_OK;
+}
+
+// Test hook, not in the header: polls of a grid barrier before it gives up.
+int avbd_test_barrier_polls(AvbdWorld* W, uint32_t polls) {
+    if (!W) return AVBD_ERR_INVALID_ARG;
+    W->polls = W->w.polls = polls;
     free_graphs(W);
     return AVBD_OK;
 }
@@ -2790,6 +2808,8 @@ int avbd_world_profile_substep(AvbdWorld* W, float* ms, uint32_t* info) {
     rc = read_ctr(W);
     if (rc) return rc;
     for (int i = 0; i < 6; i++) CK(cudaEventElapsedTime(&ms[i], ev[i], ev[i + 1]));
+    rc = timed_out(W);
+    if (rc) return rc;
     if (W->h_ctr[C_ERR]) return AVBD_ERR_CAPACITY;
     int ncol = (int)W->h_ctr[C_NCOL];
     uint32_t col_total = 0;
@@ -2825,6 +2845,8 @@ int avbd_world_profile_substep(AvbdWorld* W, float* ms, uint32_t* info) {
     ms[7] = dual;
     CK(cudaEventElapsedTime(&ms[8], ev[8], ev[9]));
     rc = read_ctr(W);
+    if (rc) return rc;
+    rc = timed_out(W);
     if (rc) return rc;
     accumulate(W);
     info[0] = (uint32_t)ncol;
@@ -2963,6 +2985,7 @@ int avbd_adjoint_backward(AvbdWorld* W, const float* grad_final, float* grad_ini
     AdjTape* t = W->adj;
     if ((uint32_t)W->w.N != t->N || (uint32_t)W->w.J != t->J || (uint32_t)W->w.S != t->S) return AVBD_ERR_INVALID_ARG;
     if (W->tune.primal_lanes != 0) return AVBD_ERR_INVALID_ARG;  // retuned since the forward
+    if (W->half_stepped) return AVBD_ERR_TIMEOUT;
     cudaSetDevice(W->device);
     cudaStream_t st = W->st;
     const int per_seg = t->every * t->substeps;
@@ -3476,6 +3499,7 @@ int avbd_snapshot_info(const void* buf, uint64_t size, AvbdSnapshotInfo* info) {
 
 int avbd_world_snapshot(AvbdWorld* W, void* buf, uint64_t cap, uint64_t* size) {
     if (!W || !size) return AVBD_ERR_INVALID_ARG;
+    if (W->half_stepped) return AVBD_ERR_TIMEOUT;
     cudaSetDevice(W->device);
     int rc = download_all(W);
     if (rc) return rc;

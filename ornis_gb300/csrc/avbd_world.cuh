@@ -320,7 +320,9 @@ struct DW {
     uint32_t* col_list;  // N: swept bodies grouped by colour, ascending index within a colour
     uint32_t *col_key, *col_key2, *col_val, *col_hist;
     uint32_t* ctr;       // counters
+    uint32_t polls;      // of a grid barrier before it gives up
 };
+constexpr uint32_t GRID_POLLS = 1u << 23;
 // The world may hold shapes whose queries are long and unlike.
 __host__ __device__ inline bool mixed_world(const DW& w) { return w.nhulls || w.nexts || w.nhfs || w.nmeshes; }
 // It may hold terrain, meshes or compounds (wide pairs).
