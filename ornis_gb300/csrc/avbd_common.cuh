@@ -4,6 +4,7 @@
 #include <cooperative_groups/reduce.h>
 
 #include "avbd_kernels.h"
+#include "avbd_resident.h"
 #include "avbd_rows.cuh"
 #include "avbd_shapes.cuh"
 
@@ -657,23 +658,18 @@ static __device__ __forceinline__ bool all_sync(const DW& w, uint32_t* bar, int 
     all_arrive(bar, kind);
     return all_wait(w, bar, kind, target, ok);
 }
-// Blocks of a kernel that the device holds at once (per device ordinal).
-struct Resident {
-    int blocks[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-};
+// Blocks of kernel k that the current device holds at once.
 template <class K>
 static int resident_blocks(Resident& r, K k, int bs, size_t smem) {
     int dev = 0;
     cudaGetDevice(&dev);
-    int& g = r.blocks[dev & 7];
-    if (!g) {
+    return r.on(dev, [&] {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0, sms = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, bs, smem);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        g = max(1, per_sm) * max(1, sms);
-    }
-    return g;
+        return max(1, per_sm) * max(1, sms);
+    });
 }
 // Launch kernel k(args..., sync kind): a block per 16 bodies (a warp of the
 // iterations per two of them: a colour is a third of a world or less), never
