@@ -126,21 +126,26 @@ static __device__ __forceinline__ void k_disc_filter_one(const DW& w, uint32_t c
     w.keep[c] = d.keep;
     if (d.keep) agg_inc_at(w.cnt, ab.x);
 }
-// New box pairs near enough to need their witness features, a warp each.
+// New box pairs near enough to need their witness features, a warp each or a
+// thread each (boxes_by_warps).
 __global__ void __launch_bounds__(128) k_disc_filter_boxes(DW w) {
     if (aborted(w)) return;
-    const uint32_t n = w.ctr[C_BOXNEW], warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
+    const uint32_t n = w.ctr[C_BOXNEW];
+    const bool warp = boxes_by_warps(w, n);
+    const uint32_t per = warp ? 32u : 1u;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / per; i < n; i += gridDim.x * blockDim.x / per) {
+        if (warp) __syncwarp();
         const uint32_t c = w.boxlist[i];
         const uint2 ab = w.cand[c];
         Disc r;
         discover_pre(w, ab.x, ab.y, r);  // passed in the filter: same state, same result
         const Shape sa = shape_of(w, ab.x), sb = shape_of(w, ab.y);
         float sat;
-        r.d = box_box_warp(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat);
+        r.d = warp ? box_box_warp(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat)
+                   : box_box(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat);
         r.sgn = sat;
         discover_post(w, ab.x, ab.y, sa, sb, r);
-        if ((threadIdx.x & 31u) == 0 && r.keep) {
+        if (r.keep && (!warp || (threadIdx.x & 31u) == 0)) {
             w.keep[c] = 1;
             atomicAdd(&w.cnt[ab.x], 1u);
         }
@@ -149,7 +154,7 @@ __global__ void __launch_bounds__(128) k_disc_filter_boxes(DW w) {
 __global__ void __launch_bounds__(128) k_disc_filter_wide(DW w) {
     if (aborted(w)) return;
     const uint32_t nw = w.ctr[C_WIDENEW];
-    const bool warp = fits_warps(nw);
+    const bool warp = fits_warps(w, nw);
     const uint32_t per = warp ? 32u : 1u;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / per; i < nw; i += gridDim.x * blockDim.x / per) {
         if (warp) __syncwarp();
@@ -221,8 +226,8 @@ __global__ void k_sort_slots(DW w) {
 static __device__ __forceinline__ bool box_pair(const DW& w, uint2 ab) {
     return info_shape(w.info[ab.x]) == AVBD_SHAPE_BOX && info_shape(w.info[ab.y]) == AVBD_SHAPE_BOX;
 }
-// Box-box witnesses are computed ahead, a warp per box pair, into bd_pa /
-// bd_pb; the per-pair build below then reads them.
+// Box-box witnesses are computed ahead, a warp or a thread per box pair
+// (boxes_by_warps), into bd_pa / bd_pb; the per-pair build below then reads them.
 // Pairs are built class by class (box-box, one box, no box) so the lanes of
 // a warp run the same manifold code: corners of two boxes, of one, or none.
 static __device__ __forceinline__ void k_collect_boxes_one(const DW& w, uint32_t p) {
@@ -242,14 +247,18 @@ __global__ void k_collect_boxes(DW w) {
 }
 __global__ void k_box_witness(DW w) {
     if (aborted(w)) return;
-    const uint32_t nbox = w.ctr[C_BOXPAIRS], warps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nbox; i += warps) {
+    const uint32_t nbox = w.ctr[C_BOXPAIRS];
+    const bool warp = boxes_by_warps(w, nbox);
+    const uint32_t per = warp ? 32u : 1u;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / per; i < nbox; i += gridDim.x * blockDim.x / per) {
+        if (warp) __syncwarp();
         uint32_t p = w.boxlist[i];
         uint2 ab = w.cand[w.slot_c[p]];
         Shape sa = shape_of(w, ab.x), sb = shape_of(w, ab.y);
         float sat;
-        Dist d = box_box_warp(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat);
-        if ((threadIdx.x & 31u) == 0) {
+        Dist d = warp ? box_box_warp(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat)
+                      : box_box(sa.pos, sa.rot, sa.p, sb.pos, sb.rot, sb.p, &sat);
+        if (!warp || (threadIdx.x & 31u) == 0) {
             w.bd_pa[p] = st3(d.pa, d.dist);
             w.bd_pb[p] = st3(d.pb, sat);
         }
@@ -423,7 +432,7 @@ __global__ void __launch_bounds__(128, 4) k_disc_build(DW w) {
 __global__ void __launch_bounds__(128, 4) k_disc_build_wide(DW w) {
     if (aborted(w)) return;
     const uint32_t n = w.ctr[C_WIDE];
-    const bool warp = fits_warps(n);
+    const bool warp = fits_warps(w, n);
     const uint32_t per = warp ? 32u : 1u;
     for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / per; i < n; i += gridDim.x * blockDim.x / per) {
         if (warp) __syncwarp();

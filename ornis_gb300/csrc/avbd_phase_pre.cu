@@ -942,7 +942,7 @@ static __device__ __forceinline__ void ccd_cast_all(const DW& w, int first, uint
     // box pairs a warp each (a cast is up to 24 distance queries in a row),
     // wide pairs too while the list is short, the rest a thread each
     const uint32_t n = w.ctr[C_FCAND], nb = w.ctr[C_FBOX], warps = gridDim.x * (blockDim.x / 32);
-    const bool wide = !WIDE || fits_warps(nb);
+    const bool wide = !WIDE || fits_warps(w, nb);
     auto is_wide = [&](uint32_t c) {
         return wide_pair(info_shape(w.info[w.cand[c].x]), info_shape(w.info[w.cand[c].y]));
     };

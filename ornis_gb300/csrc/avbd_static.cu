@@ -182,6 +182,7 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
     w.pair_cap = PCAP;
     w.max_cols = MAX_COLOURS;
     w.polls = GRID_POLLS;
+    w.warp_lists = ~0u;
     uint32_t* scene_off = cv.take<uint32_t>(S + 1);
     uint32_t* scene_of = cv.take<uint32_t>(N);
     uint32_t* plane_off = cv.take<uint32_t>(S + 1);

@@ -263,7 +263,7 @@ struct AvbdWorld {
     size_t graph_nodes = 0;       // kernel nodes in one captured substep (no events)
     size_t graph_nodes_emit = 0;  // ... in one that reports events
     uint64_t steps = 0;
-    uint32_t polls = GRID_POLLS;
+    uint32_t polls = GRID_POLLS, warp_lists = ~0u;
     bool half_stepped = false;  // a substep was cut short: no steps until a state is imported
     AdjTape* adj = nullptr;  // checkpoints of the last differentiable rollout
     uint64_t mem_gen = 0;    // bumped whenever the device arrays are (re)allocated or a launch setting changes
@@ -510,6 +510,7 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     w.enable_ccd = W->prm.enable_ccd;
     w.max_cols = MAX_COLOURS;
     w.polls = W->polls;
+    w.warp_lists = W->warp_lists;
     set_pair_ptrs(W);
     return AVBD_OK;
 }
@@ -2709,6 +2710,15 @@ int avbd_set_joint_stiffness(AvbdWorld* W, float k) {
 int avbd_test_barrier_polls(AvbdWorld* W, uint32_t polls) {
     if (!W) return AVBD_ERR_INVALID_ARG;
     W->polls = W->w.polls = polls;
+    free_graphs(W);
+    return AVBD_OK;
+}
+
+// Test hook, not in the header: the longest list of wide or box pairs that goes
+// a warp to a pair.
+int avbd_test_warp_lists(AvbdWorld* W, uint32_t n) {
+    if (!W) return AVBD_ERR_INVALID_ARG;
+    W->warp_lists = W->w.warp_lists = n;
     free_graphs(W);
     return AVBD_OK;
 }

@@ -321,6 +321,7 @@ struct DW {
     uint32_t *col_key, *col_key2, *col_val, *col_hist;
     uint32_t* ctr;       // counters
     uint32_t polls;      // of a grid barrier before it gives up
+    uint32_t warp_lists; // longest list of wide or box pairs that goes by warps
 };
 constexpr uint32_t GRID_POLLS = 1u << 23;
 // The world may hold shapes whose queries are long and unlike.
