@@ -1088,10 +1088,15 @@ void launch_ccd(const DW& w, cudaStream_t st) {
     if (!w.enable_ccd) return;
     k_ccd_collect<<<gsz(w.cand_cap, 256), 256, 0, st>>>(w);
     static Resident r, rw;
-    // a wide world's casts take up to 1 ms: a block per two bodies, where the
-    // others' small worlds gain more from a cluster's shorter start
-    if (wide_world(w)) launch_synced(rw, k_ccd_rounds<true>, 128, 0, 8 * (int)w.N, st, w);
-    else launch_synced(r, k_ccd_rounds<false>, 128, 0, w.N, st, w);
+    // A block per two bodies: a body has tens of casts in a burst, each up to 24
+    // distance queries in a row.  A block per 16, at most 8 up to 512 bodies,
+    // left 32 warps to 40,000 candidates; a substep of a burst of n boxes, ms:
+    // n = 8 0.65 -> 0.60, 128 2.99 -> 1.77, 500 11.6 -> 2.44, 1000 5.3 -> 3.1 (8.2 for
+    // the 500 with a launch per phase).  With nothing to cast the two start
+    // alike (a pile of 12 to 1500 bodies: within 0.3% either way).
+    const int per_two = 8 * (int)w.N;
+    if (wide_world(w)) launch_synced(rw, k_ccd_rounds<true>, 128, 0, per_two, st, w);
+    else launch_synced(r, k_ccd_rounds<false>, 128, 0, per_two, st, w);
 }
 
 }  // namespace avbd
