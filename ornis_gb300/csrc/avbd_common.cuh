@@ -685,12 +685,16 @@ static int resident_blocks(Resident& r, K k, int bs, size_t smem) {
 }
 // Launch kernel k(args..., sync kind): a block per 16 bodies (a warp of the
 // iterations per two of them: a colour is a third of a world or less), never
-// more than are resident.  A small world stays within the 8 blocks of a
-// portable cluster, whose barrier is the cheaper one.
+// more than are resident.  A world of up to 400 bodies stays within the 8
+// blocks of a portable cluster, whose barrier is the cheaper one; beyond, a grid
+// whose warps hold two bodies each is faster.  A substep of a pile of n boxes,
+// spheres and capsules, cluster / grid, us: n = 200 985 / 1060, 300 1170 / 1207, 400 1198 /
+// 1196, 512 1310 / 1230, 700 1431 / 1241.
+constexpr int CLUSTER_BODIES = 400;
 template <class K, class... A>
 static void launch_synced(Resident& r, K k, int bs, size_t smem, int bodies, cudaStream_t st, A... args) {
     int blocks = max(1, min(resident_blocks(r, k, bs, smem), (bodies + 15) / 16));
-    if (bodies <= 512) blocks = min(blocks, 8);
+    if (bodies <= CLUSTER_BODIES) blocks = min(blocks, 8);
     const int sync = blocks == 1 ? SYNC_BLOCK : (blocks <= 8 ? SYNC_CLUSTER : SYNC_GRID);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
