@@ -327,9 +327,11 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
         launch_iterations(w, tune, st);
         launch_finish_substep(w, tune, st);
     }
-    // Every kernel checks the error word on the device (an overflow stops the
-    // substep that met it and all later ones), so the host reads it once, with
-    // the records.
+    // A candidate overflow stops the substep that met it and all later ones on
+    // the device (aborted), so the host reads the error word once, with the
+    // records.  More colours than the solver's 64 take 2080 contacts (one at
+    // least between any two of 65 colours), more than PCAP: the candidates
+    // overflow first.
     k_static_out<<<1, MAXB, 0, st>>>(w, stage, N);
     if (cudaGetLastError() != cudaSuccess) return AVBD_ERR_DEVICE;
     uint32_t ctr[C_NUM];
@@ -338,8 +340,9 @@ extern "C" int avbd_scene_step_static(const AvbdParams* params, const AvbdBody* 
         cudaMemcpyAsync(rec, stage, sizeof(AvbdBody) * N, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return AVBD_ERR_DEVICE;
-    // more than PCAP candidates, or more colours than the solver has: out is left untouched
-    if (ctr[C_ERR] & (E_CAND_OVERFLOW | E_COLOUR_OVERFLOW)) return AVBD_ERR_CAPACITY;
+    static_assert(PCAP < (MAX_COLOURS + 1) * MAX_COLOURS / 2, "a scene of PCAP pairs could overflow the colours");
+    if (ctr[C_ERR] & E_CAND_OVERFLOW) return AVBD_ERR_CAPACITY;  // out is left untouched
+    if (ctr[C_ERR] & E_TIMEOUT) return AVBD_ERR_TIMEOUT;
     std::memcpy(out, rec, sizeof(AvbdBody) * N);
     return AVBD_OK;
 }
