@@ -58,6 +58,7 @@ struct IterRec {
 void launch_prologue(const DW& w, cudaStream_t st);
 // discovery's wake votes, wake, step-start poses and targets, contact records
 void launch_post_bodies(const DW& w, cudaStream_t st);
+constexpr int EXT_WORDS = 3;
 struct BroadphasePlan {
     const uint32_t* small_scenes = nullptr;  // device list of scenes swept by one CTA each
     int n_small = 0;
@@ -67,7 +68,7 @@ struct BroadphasePlan {
     // large scenes: sweep per row of cells in Morton order (1) or one x-sweep (0)
     int rows = 1;
     uint32_t* row_key = nullptr;  // per body of the largest scene: its row's Morton code
-    float* ext = nullptr;         // per large scene: the widest AABB edge, its sort's barrier counter
+    float* ext = nullptr;         // per large scene EXT_WORDS words (k_sap_extent)
 };
 void launch_broadphase(const DW& w, const BroadphasePlan& plan, cudaStream_t st);
 void launch_ccd(const DW& w, cudaStream_t st);

@@ -500,12 +500,13 @@ __global__ void k_sap_sweep(DW w, uint32_t n) {
 // cell coordinate, interleaved, so that neighbouring rows stay near each other;
 // rows 256 cells apart share a bucket and are told apart by their full code)
 // and, within a bucket, by min x.  A 32-bit key carries the bucket and the
-// leading 16 bits of x; bodies whose keys agree are in the order of the
-// rest of x, so a sweep ends at the first box that starts past its own
-// wherever the scene lies.  (Ordered by the key alone, 16 bits of x being steps
-// of 64 m at 10 km, 100,000 bodies at 1.4 m spacing made 194 tests a body there
-// and 814 at 100 km, against 12 at the origin: broadphase 0.47 and 0.93
-// ms.)  Each body sweeps its own row forward in the order, and the four rows of
+// leading 16 bits of x.  Where its step at the scene's farthest body is wider
+// than the widest box (row_whole_x), bodies whose keys agree are put in the
+// order of the rest of x too, and a sweep ends at the first box that starts past
+// its own: 16 bits of x are steps of 64 m at 10 km, where 100,000 bodies at 1.4 m
+// spacing made 194 tests a body by the key alone, 814 at 100 km, 13 at the
+// origin (broadphase 0.47, 0.93 and 0.18 ms; now 0.19, 0.18 and 0.13).  Nearer
+// scenes save the two passes (0.03 ms at 100,000 bodies).  Each body sweeps its own row forward in the order, and the four rows of
 // the forward half of its (y, z) neighbourhood over the x window its box can
 // reach: every overlapping pair is tested exactly once, with the same
 // closed-interval test, and the candidate set is the one-axis sweep's.  Cell
@@ -540,15 +541,23 @@ __device__ __forceinline__ void row_cells(const DW& w, uint32_t h, double cell, 
     cz = cell_of(0.5 * ((double)lo.z + (double)hi.z), cell);
 }
 // the scene's widest AABB edge (boxes are cubes here; every axis is taken)
+// ext: per large scene the widest box edge, the farthest |min x|, the sort's
+// barrier counter
+__device__ __forceinline__ bool row_whole_x(const float* ext) { return !(ext[1] * 0x1p-7f <= ext[0]); }
 __global__ void k_sap_extent(DW w, uint32_t b0, uint32_t b1, float* ext) {
-    float m = 0.0f;
+    float m = 0.0f, far = 0.0f;
     for (uint32_t h = b0 + blockIdx.x * blockDim.x + threadIdx.x; h < b1; h += gridDim.x * blockDim.x) {
         if (unbounded_kind(info_shape(w.info[h]))) continue;
         float4 lo = w.aabb_lo[h], hi = w.aabb_hi[h];
         m = fmaxf(m, fmaxf(hi.x - lo.x, fmaxf(hi.y - lo.y, hi.z - lo.z)));
+        far = fmaxf(far, fabsf(lo.x));
     }
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    for (int o = 16; o > 0; o >>= 1) {
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        far = fmaxf(far, __shfl_xor_sync(0xffffffffu, far, o));
+    }
     if ((threadIdx.x & 31) == 0 && m > 0.0f) atomicMax((int*)ext, __float_as_int(m));  // m >= 0: int order
+    if ((threadIdx.x & 31) == 0 && far > 0.0f) atomicMax((int*)ext + 1, __float_as_int(far));
 }
 // row_key: the body's row (~0 for a half-space); sort_key, x_key: its key and
 // min x, the two parts of the order
@@ -592,6 +601,8 @@ __global__ void k_sap_row_sweep(DW w, uint32_t b0, uint32_t n, const float* ext,
     if (rk == 0xffffffffu) return;  // a half-space
     const float4 alo = w.aabb_lo[a], ahi = w.aabb_hi[a];
     const uint32_t xend = x_part(ahi.x);
+    const bool whole = row_whole_x(ext);
+    const float xstop = whole ? ahi.x : INFINITY;  // boxes that start past it end a sweep
     // slots [j, ...) of the row's bucket up to the box's far side, that row only
     auto sweep = [&](uint32_t j, uint32_t row) {
         for (; j < n; j++) {
@@ -599,13 +610,13 @@ __global__ void k_sap_row_sweep(DW w, uint32_t b0, uint32_t n, const float* ext,
             if (k >> 16 != row_bucket(row) || (k & 0xffffu) > xend) break;
             const uint32_t b = w.sort_idx[j];
             const float4 blo = w.aabb_lo[b];
-            if (blo.x > ahi.x) break;
+            if (blo.x > xstop) break;
             if (row_key[b - b0] != row) continue;
             const float4 bhi = w.aabb_hi[b];
-            if (alo.x <= bhi.x && overlap_yz(alo, ahi, blo, bhi)) emit_candidate(w, a, b);
+            if (alo.x <= bhi.x && blo.x <= ahi.x && overlap_yz(alo, ahi, blo, bhi)) emit_candidate(w, a, b);
         }
     };
-    const float wmax = *ext;
+    const float wmax = ext[0];
     int cy, cz;
     row_cells(w, a, row_cell(wmax), cy, cz);
     sweep(i + 1, rk);
@@ -619,7 +630,7 @@ __global__ void k_sap_row_sweep(DW w, uint32_t b0, uint32_t n, const float* ext,
         const uint32_t row = row_code(ny, nz), key = row_bucket(row) << 16 | xbegin;
         uint32_t lo = row_lower(w.sort_key, 0, n, key);
         // many bodies of the window's first key (far from the origin): the first whose min x reaches it
-        if (lo + ROW_SKIP < n && w.sort_key[lo + ROW_SKIP] == key) {
+        if (whole && lo + ROW_SKIP < n && w.sort_key[lo + ROW_SKIP] == key) {
             uint32_t hi = row_lower(w.sort_key, lo + ROW_SKIP, n, key + 1u);
             while (lo < hi) {
                 const uint32_t m = (lo + hi) >> 1;
@@ -632,83 +643,100 @@ __global__ void k_sap_row_sweep(DW w, uint32_t b0, uint32_t n, const float* ext,
 }
 
 // ---- the rows' sort in one launch --------------------------------------------------
-// Stable LSD radix sort of (sort_key, x_key, sort_idx) in six 8-bit passes, a
-// barrier after a pass's digit counts and after its scatter: two by the low half
-// of x_key (its high half is in sort_key), which move the bodies only, then
-// four by sort_key, the first of which fetches the keys in the bodies' order.  As launches, a pass is
-// five (0.22 ms for the 45,000 bodies of a ragdoll scene, nearly all of it
-// launches and half-empty grids); here tiles are as small as gives every
-// block one, and a block adds up the counts before it itself, which is why the
-// launch form takes over above SORT_TILES tiles of 8 x 256 keys.
+// Stable LSD radix sort of (sort_key, x_key, sort_idx) in 8-bit passes, a barrier
+// after a pass's digit counts and after its scatter: two by the low half of x_key
+// (its high half is in sort_key), which move the bodies only, where row_whole_x
+// asks for them, then four by sort_key, the first of which fetches the keys in
+// the bodies' order.  As launches, a pass is five (0.22 ms for the 45,000 bodies of a
+// ragdoll scene, nearly all of it launches and half-empty grids); here tiles are
+// as small as gives every block one, and a block adds up the counts before it
+// itself, which is why the launch form takes over above SORT_TILES tiles of 8 x
+// 256 keys.  A pass is a function of its number, so that its buffers and shift
+// are constants: 100,000 bodies 15 us a pass, 26 us as a loop over passes.
 constexpr int SORT_TILES = 304;
 struct SortBufs {
     uint32_t *k0, *v0, *k1, *v1, *hist;  // k1: x_key on entry
 };
-__global__ void __launch_bounds__(256) k_sap_sort(DW w, SortBufs sb, uint32_t b0, uint32_t n, uint32_t rounds, uint32_t* bar,
-                                                  int sync) {
-    if (aborted(w)) return;
-    __shared__ uint32_t base[256], cnt[8][256], wsum[8], s_ok;
+struct SortMem {
+    uint32_t base[256], cnt[8][256], wsum[8], ok;
+};
+// One pass; false: a barrier gave up.
+template <int PASS>
+static __device__ __forceinline__ bool sort_pass(const DW& w, const SortBufs& sb, SortMem& sm, uint32_t b0, uint32_t n,
+                                                 uint32_t rounds, uint32_t* bar, int sync, uint32_t& target) {
+    constexpr int shift = PASS < 2 ? 8 * PASS : 8 * (PASS - 2);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, wid = tid >> 5, ntiles = gridDim.x;
     const uint32_t first = blockIdx.x * rounds * 256u;
-    uint32_t target = 0;
-    for (int pass = 0; pass < 6; pass++) {
-        const int shift = pass < 2 ? 8 * pass : 8 * (pass - 2);
-        const uint32_t *ki = pass & 1 ? sb.k1 : sb.k0, *vi = pass & 1 ? sb.v1 : sb.v0;
-        uint32_t *ko = pass & 1 ? sb.k0 : sb.k1, *vo = pass & 1 ? sb.v0 : sb.v1;
-        const uint32_t* by_body = pass < 2 ? sb.k1 : sb.k0;  // keys not yet moved
-        auto key_at = [&](uint32_t i) { return pass < 3 ? by_body[vi[i] - b0] : ki[i]; };
-        base[tid] = 0;
-        __syncthreads();
-        for (uint32_t r = 0; r < rounds; r++) {
-            const uint32_t i = first + r * 256u + tid;
-            if (i < n) atomicAdd(&base[(key_at(i) >> shift) & 255u], 1u);
-        }
-        __syncthreads();
-        sb.hist[blockIdx.x * 256u + tid] = base[tid];
-        if (!all_sync(w, bar, sync, target, &s_ok)) return;
-        // thread d: keys of digit d in all tiles, and in the tiles before this one
-        uint32_t total = 0, before = 0;
-        for (uint32_t t = 0; t < ntiles; t++) {
-            const uint32_t v = sb.hist[t * 256u + tid];
-            if (t < blockIdx.x) before += v;
-            total += v;
-        }
-        uint32_t inc = total;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= (uint32_t)o) inc += v;
-        }
-        if (lane == 31) wsum[wid] = inc;
-        __syncthreads();
-        uint32_t off = inc - total + before;
-        for (uint32_t k = 0; k < wid; k++) off += wsum[k];
-        base[tid] = off;
-        for (uint32_t r = 0; r < rounds; r++) {
-            for (int k = 0; k < 8; k++) cnt[k][tid] = 0;
-            __syncthreads();
-            const uint32_t i = first + r * 256u + tid;
-            const bool valid = i < n;
-            const uint32_t key = valid ? key_at(i) : 0u, d = valid ? (key >> shift) & 255u : 256u;
-            const uint32_t peers = __match_any_sync(0xffffffffu, d), rank = __popc(peers & ((1u << lane) - 1u));
-            if (valid && rank == 0) cnt[wid][d] = __popc(peers);
-            __syncthreads();
-            if (valid) {
-                uint32_t o = base[d] + rank;
-                for (uint32_t k = 0; k < wid; k++) o += cnt[k][d];
-                if (pass >= 2) ko[o] = key;
-                vo[o] = vi[i];
-            }
-            __syncthreads();
-            uint32_t add = 0;
-            for (int k = 0; k < 8; k++) add += cnt[k][tid];
-            base[tid] += add;
-            __syncthreads();
-        }
-        if (pass < 5 && !all_sync(w, bar, sync, target, &s_ok)) return;
+    const uint32_t *ki = PASS & 1 ? sb.k1 : sb.k0, *vi = PASS & 1 ? sb.v1 : sb.v0;
+    uint32_t *ko = PASS & 1 ? sb.k0 : sb.k1, *vo = PASS & 1 ? sb.v0 : sb.v1;
+    const uint32_t* by_body = PASS < 2 ? sb.k1 : sb.k0;  // keys not yet moved
+    auto key_at = [&](uint32_t i) { return PASS < 3 ? by_body[vi[i] - b0] : ki[i]; };
+    sm.base[tid] = 0;
+    __syncthreads();
+    for (uint32_t r = 0; r < rounds; r++) {
+        const uint32_t i = first + r * 256u + tid;
+        if (i < n) atomicAdd(&sm.base[(key_at(i) >> shift) & 255u], 1u);
     }
+    __syncthreads();
+    sb.hist[blockIdx.x * 256u + tid] = sm.base[tid];
+    if (!all_sync(w, bar, sync, target, &sm.ok)) return false;
+    // thread d: keys of digit d in all tiles, and in the tiles before this one
+    uint32_t total = 0, before = 0;
+    for (uint32_t t = 0; t < ntiles; t++) {
+        const uint32_t v = sb.hist[t * 256u + tid];
+        if (t < blockIdx.x) before += v;
+        total += v;
+    }
+    uint32_t inc = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += v;
+    }
+    if (lane == 31) sm.wsum[wid] = inc;
+    __syncthreads();
+    uint32_t off = inc - total + before;
+    for (uint32_t k = 0; k < wid; k++) off += sm.wsum[k];
+    sm.base[tid] = off;
+    for (uint32_t r = 0; r < rounds; r++) {
+        for (int k = 0; k < 8; k++) sm.cnt[k][tid] = 0;
+        __syncthreads();
+        const uint32_t i = first + r * 256u + tid;
+        const bool valid = i < n;
+        const uint32_t key = valid ? key_at(i) : 0u, d = valid ? (key >> shift) & 255u : 256u;
+        const uint32_t peers = __match_any_sync(0xffffffffu, d), rank = __popc(peers & ((1u << lane) - 1u));
+        if (valid && rank == 0) sm.cnt[wid][d] = __popc(peers);
+        __syncthreads();
+        if (valid) {
+            uint32_t o = sm.base[d] + rank;
+            for (uint32_t k = 0; k < wid; k++) o += sm.cnt[k][d];
+            if (PASS >= 2) ko[o] = key;
+            vo[o] = vi[i];
+        }
+        __syncthreads();
+        uint32_t add = 0;
+        for (int k = 0; k < 8; k++) add += sm.cnt[k][tid];
+        sm.base[tid] += add;
+        __syncthreads();
+    }
+    return PASS == 5 || all_sync(w, bar, sync, target, &sm.ok);
 }
-static void launch_row_sort(const DW& w, const BroadphasePlan& plan, uint32_t b0, uint32_t n, uint32_t* bar, cudaStream_t st) {
+__global__ void __launch_bounds__(256) k_sap_sort(DW w, SortBufs sb, uint32_t b0, uint32_t n, uint32_t rounds, float* ext,
+                                                  int sync) {
+    if (aborted(w)) return;
+    __shared__ SortMem sm;
+    uint32_t* bar = (uint32_t*)(ext + 2);
+    uint32_t target = 0;
+    if (row_whole_x(ext)) {
+        if (!sort_pass<0>(w, sb, sm, b0, n, rounds, bar, sync, target)) return;
+        if (!sort_pass<1>(w, sb, sm, b0, n, rounds, bar, sync, target)) return;
+    }
+    if (!sort_pass<2>(w, sb, sm, b0, n, rounds, bar, sync, target)) return;
+    if (!sort_pass<3>(w, sb, sm, b0, n, rounds, bar, sync, target)) return;
+    if (!sort_pass<4>(w, sb, sm, b0, n, rounds, bar, sync, target)) return;
+    sort_pass<5>(w, sb, sm, b0, n, rounds, bar, sync, target);
+}
+static void launch_row_sort(const DW& w, const BroadphasePlan& plan, uint32_t b0, uint32_t n, float* ext, cudaStream_t st) {
     static Resident r;
     const uint32_t rounds = (n + SORT_TILES * 256u - 1) / (SORT_TILES * 256u);
     const uint32_t tiles = (n + rounds * 256u - 1) / (rounds * 256u);
@@ -728,7 +756,7 @@ static void launch_row_sort(const DW& w, const BroadphasePlan& plan, uint32_t b0
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k_sap_sort, w, SortBufs{w.sort_key, w.sort_idx, plan.keys_alt, plan.vals_alt, plan.hist}, b0, n,
-                       rounds, bar, (int)SYNC_GRID);
+                       rounds, ext, (int)SYNC_GRID);
 }
 
 // Swept-cast state of body h, and the list of the fast bodies.
@@ -793,16 +821,15 @@ void launch_broadphase(const DW& w, const BroadphasePlan& plan, cudaStream_t st)
         k_sap_small<<<plan.n_small, 512, 0, st>>>(w, plan.small_scenes, plan.n_small);
         k_sap_small_sweep<<<gsz((size_t)w.N * 32, 256), 256, 0, st>>>(w, plan.small_max);
     }
-    // per large scene its widest box edge and its sort's barrier counter
-    if (plan.rows && !plan.large.empty()) cudaMemsetAsync(plan.ext, 0, plan.large.size() * 2 * sizeof(float), st);
+    if (plan.rows && !plan.large.empty()) cudaMemsetAsync(plan.ext, 0, plan.large.size() * EXT_WORDS * sizeof(float), st);
     for (size_t i = 0; i < plan.large.size(); i++) {
         uint32_t b0 = plan.large[i].first, b1 = plan.large[i].second;
         uint32_t n = b1 - b0;
         if (plan.rows) {
-            float* ext = plan.ext + 2 * i;
+            float* ext = plan.ext + EXT_WORDS * i;
             k_sap_extent<<<std::min<unsigned>(nblk(n, 256), 4u * 152u), 256, 0, st>>>(w, b0, b1, ext);
             k_sap_row_keys<<<nblk(n, 256), 256, 0, st>>>(w, b0, b1, ext, plan.row_key, plan.keys_alt);
-            launch_row_sort(w, plan, b0, n, (uint32_t*)(ext + 1), st);
+            launch_row_sort(w, plan, b0, n, ext, st);
             k_sap_row_sweep<<<nblk(n, 128), 128, 0, st>>>(w, b0, n, ext, plan.row_key);
             continue;
         }

@@ -424,7 +424,7 @@ static int alloc_device(AvbdWorld* W, uint32_t N, uint32_t J, uint32_t cand_cap)
     W->plan.hist = m.get<uint32_t>(std::max<size_t>(radix_hist_words(max_large), SORT_HIST_WORDS));
     W->plan.rows = W->tune.sweep_rows;
     W->plan.row_key = m.get<uint32_t>(max_large);
-    W->plan.ext = m.get<float>(2 * W->plan.large.size());
+    W->plan.ext = m.get<float>(EXT_WORDS * W->plan.large.size());
     size_t scan_words = std::max({SCAN_MANY * scan_tmp_words((size_t)N + 1), scan_tmp_words(radix_hist_words(max_large)),
                                   scan_tmp_words(radix_hist_words(N))});
     W->scan_tmp = m.get<uint32_t>(scan_words + 16);

@@ -39,7 +39,7 @@ def both_sweeps(bodies, steps):
     assert out[0] == out[1]
 
 
-@pytest.mark.parametrize("shift", [-1e4, 3e3, 1e5])
+@pytest.mark.parametrize("shift", [0.0, 60.0, 300.0, -1e4, 3e3, 1e5])
 def test_candidates_away_from_the_origin(shift):
     both_sweeps(field(4000, shift, pitch=1.1), 3)
 
