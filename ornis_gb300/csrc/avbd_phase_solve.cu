@@ -1079,8 +1079,10 @@ __global__ void __launch_bounds__(256) k_entries(DW w) {
             np = min(w.p_np[p], (uint32_t)MAX_PTS);
             const uint2 ab = w.p_ab[p];
             other = side_a ? ab.y : ab.x;
-            const int co = w.colour[other];
-            dual = co < 0 || w.colour[h] < co;
+            // neighbours have one colour only where the scene has more than the
+            // solver's 64 (E_COLOUR_OVERFLOW): the lower handle's side then
+            const int ch = w.colour[h], co = w.colour[other];
+            dual = co < 0 || ch < co || (ch == co && h < other);
             if (w.p_n[p].w <= 0.0f) {
                 const float4 ma = w.mat[ab.x], mb = w.mat[ab.y];
                 roll = fmaxf(ma.z, mb.z) > 0.0f || fmaxf(ma.w, mb.w) > 0.0f;
